@@ -9,6 +9,7 @@
 #include <mutex>
 
 #include "host.h"
+#include "mma8.h"
 #include "tune_table.h"
 
 namespace kcv {
@@ -465,12 +466,16 @@ cudaError_t upload_async(kleidicv_gpu_context *ctx, void *dst, const void *src, 
   return cudaEventRecord(u.done, ctx->stream);
 }
 
-void *ctx_alloc(kleidicv_gpu_context *ctx, size_t bytes) {
+bool ctx_admits(kleidicv_gpu_context *ctx, size_t bytes) {
   int f = ctx->fail_allocs.load();
   while (f > 0) {
-    if (ctx->fail_allocs.compare_exchange_weak(f, f - 1)) return nullptr;
+    if (ctx->fail_allocs.compare_exchange_weak(f, f - 1)) return false;
   }
-  if (ctx->pool_used.load() + bytes > ctx->pool_limit) return nullptr;
+  return ctx->pool_used.load() + bytes <= ctx->pool_limit;
+}
+
+void *ctx_alloc(kleidicv_gpu_context *ctx, size_t bytes) {
+  if (!ctx_admits(ctx, bytes)) return nullptr;
   void *p = nullptr;
   if (cudaMallocAsync(&p, bytes, ctx->stream) != cudaSuccess) return nullptr;
   ctx->pool_used += bytes;
@@ -528,6 +533,13 @@ kleidicv_error_t execute(kleidicv_gpu_context *ctx, Prepared &p) {
         ctx->launches += 1;
         return cuda_status(ctx, launch_gauss8(p.fused, ctx->sm_count, ctx->stream));
       }
+      Mma8Job mj;
+      if (ctx->tune_threads <= 0 && mma8_job(p.fused, ctx->sm_count, mj)) {
+        // Other generated Gaussians and the u8 separable filter: the
+        // tensor-core stencil of mma8.cuh.
+        ctx->launches += 1;
+        return cuda_status(ctx, launch_mma8(mj, ctx->sm_count, ctx->stream));
+      }
       if (ctx->tune_threads <= 0 && sep16_eligible(p.fused)) {
         // One-channel 16-bit 5x5: the fp32 streaming kernel of sep16.cu.
         ctx->launches += 1;
@@ -578,6 +590,13 @@ kleidicv_error_t execute(kleidicv_gpu_context *ctx, Prepared &p) {
       const GenericJob &g = p.generic;
       const size_t vstride = (static_cast<size_t>(g.width) * g.channels + 15) / 16 * 16;
       const size_t bytes = vstride * g.height;
+      Mma8Job mj;
+      if (mma8_job(g, ctx->sm_count, mj)) {
+        // Nothing is allocated, but a call that the pool cap refuses stays refused.
+        if (!ctx_admits(ctx, bytes)) return KLEIDICV_ERROR_ALLOCATION;
+        ctx->launches += 1;
+        return cuda_status(ctx, launch_mma8(mj, ctx->sm_count, ctx->stream));
+      }
       uint8_t *scratch = static_cast<uint8_t *>(ctx_alloc(ctx, bytes));
       if (!scratch) return KLEIDICV_ERROR_ALLOCATION;
       cudaError_t e = launch_generic_gaussian(g, scratch, vstride, ctx->stream);

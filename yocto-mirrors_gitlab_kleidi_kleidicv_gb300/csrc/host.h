@@ -139,6 +139,8 @@ void shutdown_async(kleidicv_gpu_context *ctx);
 
 // Context helpers.
 kleidicv_error_t resolve_context(kleidicv_gpu_context *&ctx);
+// Whether the pool cap (and the injected failures) allow `bytes` more.
+bool ctx_admits(kleidicv_gpu_context *ctx, size_t bytes);
 void *ctx_alloc(kleidicv_gpu_context *ctx, size_t bytes);
 void ctx_free(kleidicv_gpu_context *ctx, void *p, size_t bytes);
 // Copies `bytes` from host memory `src` to device memory `dst` on the

@@ -130,6 +130,32 @@ struct Gauss8Job {
   int32_t item_end;        // batch tables: items of this and the earlier entries
 };
 
+// u8 separable stencils on the tensor cores (csrc/mma8.cuh): generated
+// Gaussians of any size and the u8 separable filter.  A tile is 16 * MT
+// destination rows x tile_w destination bytes.
+struct Mma8Job {
+  const uint8_t *src;
+  uint8_t *dst;
+  int64_t src_stride, dst_stride;  // bytes
+  int32_t w, h, c, wc;             // pixels, rows, channels, bytes per row
+  int32_t border, border_value;
+  int32_t ksize, r, rc;   // taps, taps on either side, bytes on either side
+  int32_t hp, vo;         // rc rounded up to 16 (halo of the staged source) and to 4 (of V)
+  // Contraction steps: 16 source rows for 8 destination rows; 16 bytes of V
+  // for destination bytes 8..15 (nb) and 0..7 (na) of 16.
+  int32_t nk, nb, na;
+  int32_t mt, tile_w;     // a tile: 16 mt rows (1, 2, 4), destination bytes (a multiple of 128)
+  int32_t epi;            // Mma8Epi
+  int32_t tiles_x, tiles_y;
+  int32_t raw_rows, raw_cols, raw_pitch;  // staged source: rows, bytes at a time, bytes between rows
+  int32_t v_cols, v_pitch;                // vertical results
+  // kEpiArbitrary: vertical sums saturate; horizontal sums of these bytes of a
+  // row saturate; the right-border lanes of rows of several channels.
+  int32_t saturate, h_sat_from, h_sat_to, quirk, arb_border_len;
+  int32_t smem_bytes;
+  uint8_t ty[256], tx[256];  // taps of the passes
+};
+
 // Blur-and-downsample levels (csrc/pyramid.cu).  One entry is one level of
 // one image: src (w x h) -> dst ((w+1)/2 x (h+1)/2), computed in warp items:
 // first its edge tasks (32 edge elements each), then (strip of 32 lanes of

@@ -1,0 +1,36 @@
+// Host interface of the tensor-core u8 stencils (mma8.cuh, mma8*.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "kcv_job.h"
+
+namespace kcv {
+
+// Fills the job of a fused Gaussian with generated weights or a u8 separable
+// filter, or of an arbitrary-size Gaussian, tiled for `sm_count` SMs.  False:
+// the call is not of these kinds (or overlaps its source), and the job is not
+// filled.
+bool mma8_job(const FilterJob &f, int sm_count, Mma8Job &j);
+bool mma8_job(const GenericJob &g, int sm_count, Mma8Job &j);
+cudaError_t launch_mma8(const Mma8Job &j, int sm_count, cudaStream_t stream);
+
+// Instantiations, one translation unit each: <vertical steps>_<horizontal
+// steps nb>_<na>, or any number of steps; the u8 separable filter.
+cudaError_t launch_mma8_1_2_1(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_1_2_2(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_1_3_2(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_1_3_3(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_2_2_2(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_2_3_2(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_2_3_3(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_2_4_4(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_2_5_4(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_3_3_3(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_3_4_3(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_2_any(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_3_any(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_0_any(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_sat8(const Mma8Job &j, int sm_count, cudaStream_t stream);
+
+}  // namespace kcv

@@ -1,0 +1,10 @@
+// Tensor-core stencil: 11 to 25 taps, horizontal windows of 3 and 3 blocks.
+#include "mma8_launch.cuh"
+
+namespace kcv {
+
+cudaError_t launch_mma8_2_3_3(const Mma8Job &j, int sm_count, cudaStream_t stream) {
+  return launch_mma8_tiled<2, 3, 3, kEpiRound>(j, sm_count, stream);
+}
+
+}  // namespace kcv

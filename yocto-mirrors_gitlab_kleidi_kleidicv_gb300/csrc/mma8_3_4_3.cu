@@ -1,0 +1,10 @@
+// Tensor-core stencil: 27 to 41 taps, horizontal windows of 4 and 3 blocks.
+#include "mma8_launch.cuh"
+
+namespace kcv {
+
+cudaError_t launch_mma8_3_4_3(const Mma8Job &j, int sm_count, cudaStream_t stream) {
+  return launch_mma8_tiled<3, 4, 3, kEpiRound>(j, sm_count, stream);
+}
+
+}  // namespace kcv

@@ -42,4 +42,34 @@ cudaError_t resident_ctas_per_sm(int threads, int smem, int *per_sm) {
   return cudaSuccess;
 }
 
+// The same with the register and thread limits alone: raises the dynamic
+// shared-memory limit to `max_smem` and returns how many CTAs would fit if
+// each took no shared memory (kernels whose shared memory varies by job).
+template <auto Kern>
+cudaError_t resident_by_registers(int threads, int max_smem, int *per_sm) {
+  constexpr int kDevices = 64;
+  static std::atomic<int> cached[kDevices];  // zero-initialised: not yet known
+  static std::mutex m;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= kDevices) return cudaErrorInvalidDevice;
+  int v = cached[dev].load(std::memory_order_acquire);
+  if (v == 0) {
+    std::lock_guard<std::mutex> lock(m);
+    v = cached[dev].load(std::memory_order_relaxed);
+    if (v == 0) {
+      e = cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+      if (e != cudaSuccess) return e;
+      int occ = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, Kern, threads, 0);
+      if (e != cudaSuccess) return e;
+      v = occ > 1 ? occ : 1;
+      cached[dev].store(v, std::memory_order_release);
+    }
+  }
+  *per_sm = v;
+  return cudaSuccess;
+}
+
 }  // namespace kcv
