@@ -111,3 +111,32 @@ def test_in_place_arbitrary_size_keeps_its_result():
     assert ctx.synchronize() == kcv.OK
     ctx.close()
     assert np.array_equal(img.cpu().numpy(), oracle.gaussian_blur_u8(host, w, h, c, k, 4.0, kcv.REPLICATE)[1])
+
+
+def test_batch_runs_of_tiles():
+    """A plan whose jobs hold one tile, several and more than a CTA's run, of
+    every instantiation, twice (the second launch replays the graph)."""
+    rng = np.random.default_rng(77)
+    items, reqs = [], []
+    for n, (k, c) in enumerate([s for s in STEPS if s[0] <= 15] * 3):
+        w, h = ((2500 // c, 700), (20, 15), (256 // c + 1, 129))[n % 3]
+        host = rng.integers(0, 256, (h, w * c + n % 5), dtype=np.uint8)
+        sbuf, sptr, sstride = device_image(torch, host)
+        dbuf, dptr, dstride = device_output(torch, h, w * c, np.uint8, pad_elems=n % 4)
+        border = FIXED[n % 4]
+        reqs.append(kcv.make_request(kcv.OP_GAUSSIAN_BLUR_U8, sptr, sstride, dptr, dstride, w, h, c, k, k, 1.4, 1.4,
+                                     border_type=border))
+        items.append((sbuf, dbuf, dstride, w, h, c, oracle.gaussian_blur_u8(host, w, h, c, k, 1.4, border)[1]))
+    ctx = kcv.Context.for_torch(0)
+    plan = kcv.BatchPlan(reqs, ctx)
+    assert plan.statuses == [kcv.OK] * len(reqs)
+    for _ in range(2):
+        for it in items:
+            it[1].fill_(0xA5)
+        assert plan.launch(True) == kcv.OK
+        assert ctx.synchronize() == kcv.OK
+        for _, dbuf, dstride, w, h, c, want in items:
+            got, pad_ok = read_output(dbuf, h, w * c, np.uint8, dstride)
+            assert pad_ok and np.array_equal(got, want), (w, h, c)
+    plan.close()
+    ctx.close()

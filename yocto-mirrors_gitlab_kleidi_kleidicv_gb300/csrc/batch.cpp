@@ -8,13 +8,16 @@
 // (mode, size, channels), orders each group's tiles largest first, and
 // uploads the job table and the work-lists in one device allocation.  A
 // launch resets the work counters and starts one persistent kernel per group
-// on forked streams, so the groups run concurrently; blur-and-downsample
-// requests go to the pyramid kernel and four-channel generated 3x3 / 5x5 /
-// 7x7 Gaussians to the streaming kernel of gauss8.cu (one launch per channel
-// count or kernel size, over an entry table), and arbitrary-size Gaussians
-// (two-pass kernel with a scratch image) and copies run on a branch of their
-// own.  With use_graph the whole
-// launch is captured once into a CUDA graph and replayed.
+// on forked streams, so the groups run concurrently.  Blur-and-downsample
+// requests go to the pyramid kernel, four-channel generated 3x3 / 5x5 / 7x7
+// Gaussians to the streaming kernel of gauss8.cu and the other generated
+// Gaussians up to 15 taps and the u8 separable filter to the tensor-core
+// stencil of mma8.cuh (one launch per channel count, kernel size or
+// instantiation, over a job table): 512 images of 64..4096 x 64..2160 and 3 to
+// 15 taps 2373 -> 1056 us.  On the stencil the four-channel 3 / 5 / 7 taps of
+// that batch alone take 133 / 124 / 138 us against 75 / 75 / 109 us.
+// Arbitrary-size Gaussians and copies run on a branch of their own.  With
+// use_graph the whole launch is captured once into a CUDA graph and replayed.
 #include <string.h>
 
 #include <algorithm>
@@ -23,6 +26,7 @@
 #include <vector>
 
 #include "host.h"
+#include "mma8.h"
 
 namespace kcv {
 namespace {
@@ -105,6 +109,15 @@ struct kleidicv_gpu_batch_plan {
   // Four-channel generated Gaussians by kernel size (index (K - 3) / 2).
   std::vector<kcv::Gauss8Job> g8[3];
   kcv::Gauss8Job *d_g8[3] = {nullptr, nullptr, nullptr};
+  // Tensor-core stencil jobs by instantiation (mma8_batch_key).
+  struct Mma8Group {
+    std::vector<kcv::Mma8Job> jobs;
+    std::vector<int> ends;
+    long tiles = 0;
+    kcv::Mma8Batch batch{};
+  };
+  std::map<int, Mma8Group> mma8;
+  int *d_mma8_next = nullptr;
   uint8_t *dmem = nullptr;
   size_t dmem_bytes = 0;
   FilterJob *d_jobs = nullptr;
@@ -112,6 +125,9 @@ struct kleidicv_gpu_batch_plan {
   int *d_next = nullptr;
   std::vector<Group> groups;
   std::vector<FilterJob> jobs;
+  // Arbitrary-size Gaussians: on the tensor-core stencil, or (in-place calls)
+  // with a scratch image on the two-pass kernel.
+  std::vector<Mma8Job> arbitrary;
   std::vector<GenericJob> generic;
   std::vector<size_t> generic_off, generic_stride;
   std::vector<Prepared> copies;
@@ -129,6 +145,7 @@ kleidicv_error_t enqueue(kleidicv_gpu_batch_plan *p, cudaStream_t s) {
   kleidicv_gpu_context *ctx = p->ctx;
   cudaError_t e = cudaSuccess;
   if (!p->groups.empty()) e = cudaMemsetAsync(p->d_next, 0, p->groups.size() * sizeof(int), s);
+  if (e == cudaSuccess && !p->mma8.empty()) e = cudaMemsetAsync(p->d_mma8_next, 0, p->mma8.size() * sizeof(int), s);
   if (e == cudaSuccess) e = cudaEventRecord(p->fork, s);
   const size_t nb = p->branches.size();
   std::vector<bool> used(nb, false);
@@ -136,6 +153,12 @@ kleidicv_error_t enqueue(kleidicv_gpu_batch_plan *p, cudaStream_t s) {
   // Groups round-robin over the branches; the last branch also takes the
   // generic jobs and copies.
   size_t lane = 0;  // next branch, round robin
+  for (auto &m : p->mma8) {
+    if (e != cudaSuccess) break;
+    const size_t b = nb ? lane++ % nb : 0;
+    used[b] = true;
+    e = launch_mma8_batch(m.second.jobs[0], m.second.batch, ctx->sm_count, nb ? p->branches[b] : s);
+  }
   for (size_t g = 0; g < p->groups.size() && e == cudaSuccess; ++g, ++lane) {
     const Group &gr = p->groups[g];
     BatchLaunch bl{p->d_jobs, p->d_tiles + gr.tile_off, gr.ntiles, p->d_next + g, gr.smem, gr.grid};
@@ -165,6 +188,10 @@ kleidicv_error_t enqueue(kleidicv_gpu_batch_plan *p, cudaStream_t s) {
                             ctx->sm_count, nb ? p->branches[b] : s);
   }
   cudaStream_t tail = nb ? p->branches[nb - 1] : s;
+  for (size_t i = 0; i < p->arbitrary.size() && e == cudaSuccess; ++i) {
+    e = launch_mma8(p->arbitrary[i], ctx->sm_count, tail);
+    if (nb) used[nb - 1] = true;
+  }
   for (size_t i = 0; i < p->generic.size() && e == cudaSuccess; ++i) {
     e = launch_generic_gaussian(p->generic[i], p->dmem + p->generic_off[i], p->generic_stride[i], tail);
     if (nb) used[nb - 1] = true;
@@ -201,7 +228,7 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
 
   std::map<std::tuple<int, int, int, int>, size_t> group_of;
   long g8_items_bound[3] = {0, 0, 0};
-  size_t generic_bytes = 0;
+  size_t generic_bytes = 0, admitted_bytes = 0;
   for (size_t i = 0; i < count; ++i) {
     Prepared pr;
     const kleidicv_error_t st = prepare_request(requests[i], &pr);
@@ -216,6 +243,13 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
       case Prepared::GENERIC: {
         const GenericJob &g = pr.generic;
         const size_t stride = align_up(static_cast<size_t>(g.width) * g.channels, 16);
+        Mma8Job m;
+        if (mma8_job(g, ctx->sm_count, m)) {
+          // No scratch image, but a plan that the pool cap refuses stays refused.
+          p->arbitrary.push_back(m);
+          admitted_bytes += align_up(stride * g.height, 256);
+          break;
+        }
         p->generic.push_back(g);
         p->generic_stride.push_back(stride);
         p->generic_off.push_back(generic_bytes);  // relative; rebased below
@@ -234,6 +268,21 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
             gauss8_job(pr.fused, g);  // bands sized once the request count is known
             p->g8[k].push_back(g);
             break;
+          }
+        }
+        {
+          // Tile counts of a table stay in 32 bits.
+          Mma8Job m;
+          if (mma8_batch_job(pr.fused, m) && mma8_batch_key(m) != 0) {
+            auto &gr = p->mma8[mma8_batch_key(m)];
+            const long tiles = static_cast<long>(m.tiles_x) * m.tiles_y;
+            if (gr.tiles + tiles < (1L << 30)) {
+              gr.tiles += tiles;
+              gr.jobs.push_back(m);
+              gr.ends.push_back(static_cast<int>(gr.tiles));
+              break;
+            }
+            if (gr.jobs.empty()) p->mma8.erase(mma8_batch_key(m));
           }
         }
         if (pr.fused.mode == MODE_BLURDOWN) {
@@ -336,8 +385,19 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
   const size_t next_bytes = align_up(p->groups.size() * sizeof(int), 256);
   const size_t pyr_total = pyr_bytes[0] + pyr_bytes[1] + pyr_bytes[2] + pyr_bytes[3];
   const size_t g8_total = g8_bytes[0] + g8_bytes[1] + g8_bytes[2];
-  p->dmem_bytes = jobs_bytes + tiles_bytes + next_bytes + generic_bytes + pyr_total + g8_total;
-  if (p->dmem_bytes) {
+  size_t mma8_total = p->mma8.empty() ? 0 : align_up(p->mma8.size() * sizeof(int), 256);
+  for (auto &m : p->mma8) {
+    mma8_total += align_up(m.second.jobs.size() * sizeof(Mma8Job), 256) +
+                  align_up(m.second.ends.size() * sizeof(int), 256);
+    p->tiles_total += m.second.tiles;
+  }
+  p->dmem_bytes = jobs_bytes + tiles_bytes + next_bytes + generic_bytes + pyr_total + g8_total + mma8_total;
+  if (admitted_bytes && ctx->pool_used.load() + p->dmem_bytes + admitted_bytes > ctx->pool_limit) {
+    delete p;
+    return KLEIDICV_ERROR_ALLOCATION;
+  }
+  if (p->dmem_bytes || admitted_bytes) {
+    if (p->dmem_bytes == 0) p->dmem_bytes = 256;
     p->dmem = static_cast<uint8_t *>(ctx_alloc(ctx, p->dmem_bytes));
     if (!p->dmem) {
       delete p;
@@ -360,6 +420,21 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
       p->d_g8[k] = reinterpret_cast<Gauss8Job *>(p->dmem + off);
       off += g8_bytes[k];
     }
+    // The counters, then each group's jobs and tile ends.
+    p->d_mma8_next = reinterpret_cast<int *>(p->dmem + off);
+    if (!p->mma8.empty()) off += align_up(p->mma8.size() * sizeof(int), 256);
+    int k = 0;
+    for (auto &m : p->mma8) {
+      Mma8Batch &b = m.second.batch;
+      b.jobs = reinterpret_cast<const Mma8Job *>(p->dmem + off);
+      off += align_up(m.second.jobs.size() * sizeof(Mma8Job), 256);
+      b.ends = reinterpret_cast<const int *>(p->dmem + off);
+      off += align_up(m.second.ends.size() * sizeof(int), 256);
+      b.n = static_cast<int>(m.second.jobs.size());
+      b.tiles = static_cast<int>(m.second.tiles);
+      b.next = p->d_mma8_next + k++;
+      b.smem_bytes = m.second.jobs[0].smem_bytes;  // of the instantiation
+    }
   }
   // Through the pinned upload ring: no wait for the stream's earlier work.
   cudaError_t ce = upload_async(ctx, p->d_jobs, p->jobs.data(), p->jobs.size() * sizeof(FilterJob));
@@ -369,8 +444,14 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
     if (p->d_pyr[c]) ce = upload_async(ctx, p->d_pyr[c], p->pyr[c].data(), p->pyr[c].size() * sizeof(PyrEntry));
   for (int k = 0; k < 3 && ce == cudaSuccess; ++k)
     if (p->d_g8[k]) ce = upload_async(ctx, p->d_g8[k], p->g8[k].data(), p->g8[k].size() * sizeof(Gauss8Job));
-  const size_t nbranch = std::min<size_t>(kMaxBranches, p->groups.size() + npyr_groups + ng8_groups +
-                                          ((p->generic.empty() && p->copies.empty()) ? 0 : 1));
+  for (auto &m : p->mma8) {
+    const Mma8Batch &b = m.second.batch;
+    if (ce == cudaSuccess)
+      ce = upload_async(ctx, const_cast<Mma8Job *>(b.jobs), m.second.jobs.data(), b.n * sizeof(Mma8Job));
+    if (ce == cudaSuccess) ce = upload_async(ctx, const_cast<int *>(b.ends), m.second.ends.data(), b.n * sizeof(int));
+  }
+  const size_t nbranch = std::min<size_t>(kMaxBranches, p->groups.size() + npyr_groups + ng8_groups + p->mma8.size() +
+                                          ((p->arbitrary.empty() && p->generic.empty() && p->copies.empty()) ? 0 : 1));
   if (ce == cudaSuccess) {
     // The context's branch streams and events, created once and shared.
     std::lock_guard<std::mutex> lock(ctx->branch_mutex);
@@ -394,7 +475,8 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
       p->joins.assign(ctx->branch_events.begin(), ctx->branch_events.begin() + nbranch);
     }
   }
-  p->kernels_per_launch = p->groups.size() + npyr_groups + ng8_groups + 2 * p->generic.size();
+  p->kernels_per_launch = p->groups.size() + npyr_groups + ng8_groups + p->mma8.size() + p->arbitrary.size() +
+                          2 * p->generic.size();
   if (ce != cudaSuccess) {
     kleidicv_gpu_batch_plan_destroy(p);
     return cuda_status(ctx, ce);

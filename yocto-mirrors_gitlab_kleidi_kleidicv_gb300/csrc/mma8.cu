@@ -119,25 +119,45 @@ bool mma8_job(const GenericJob &g, int sm_count, Mma8Job &j) {
   return plan(j, sm_count);
 }
 
-cudaError_t launch_mma8(const Mma8Job &j, int sm_count, cudaStream_t stream) {
-  if (j.epi == kEpiSat8) return launch_mma8_sat8(j, sm_count, stream);
-  if (fixed_steps(j)) {
-    switch (100 * j.nk + 10 * j.nb + j.na) {
-      case 121: return launch_mma8_1_2_1(j, sm_count, stream);
-      case 122: return launch_mma8_1_2_2(j, sm_count, stream);
-      case 132: return launch_mma8_1_3_2(j, sm_count, stream);
-      case 133: return launch_mma8_1_3_3(j, sm_count, stream);
-      case 222: return launch_mma8_2_2_2(j, sm_count, stream);
-      case 232: return launch_mma8_2_3_2(j, sm_count, stream);
-      case 233: return launch_mma8_2_3_3(j, sm_count, stream);
-      case 244: return launch_mma8_2_4_4(j, sm_count, stream);
-      case 254: return launch_mma8_2_5_4(j, sm_count, stream);
-      case 333: return launch_mma8_3_3_3(j, sm_count, stream);
-      case 343: return launch_mma8_3_4_3(j, sm_count, stream);
-    }
+namespace {
+
+// Instantiations with both step counts at compile time.
+cudaError_t launch_fixed(const Mma8Job &j, const Mma8Batch *batch, int sm_count, cudaStream_t stream) {
+  if (j.epi == kEpiSat8) return launch_mma8_sat8(j, batch, sm_count, stream);
+  switch (mma8_batch_key(j)) {
+    case 121: return launch_mma8_1_2_1(j, batch, sm_count, stream);
+    case 122: return launch_mma8_1_2_2(j, batch, sm_count, stream);
+    case 132: return launch_mma8_1_3_2(j, batch, sm_count, stream);
+    case 133: return launch_mma8_1_3_3(j, batch, sm_count, stream);
+    case 222: return launch_mma8_2_2_2(j, batch, sm_count, stream);
+    case 232: return launch_mma8_2_3_2(j, batch, sm_count, stream);
+    case 233: return launch_mma8_2_3_3(j, batch, sm_count, stream);
+    case 244: return launch_mma8_2_4_4(j, batch, sm_count, stream);
+    case 254: return launch_mma8_2_5_4(j, batch, sm_count, stream);
+    case 333: return launch_mma8_3_3_3(j, batch, sm_count, stream);
+    case 343: return launch_mma8_3_4_3(j, batch, sm_count, stream);
   }
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace
+
+cudaError_t launch_mma8(const Mma8Job &j, int sm_count, cudaStream_t stream) {
+  if (fixed_steps(j)) return launch_fixed(j, nullptr, sm_count, stream);
   if (j.nk <= 2) return launch_mma8_2_any(j, sm_count, stream);
   return j.nk == 3 ? launch_mma8_3_any(j, sm_count, stream) : launch_mma8_0_any(j, sm_count, stream);
+}
+
+int mma8_batch_key(const Mma8Job &j) {
+  if (!fixed_steps(j)) return 0;
+  return 1000 * (j.epi == kEpiSat8) + 100 * j.nk + 10 * j.nb + j.na;
+}
+
+bool mma8_batch_job(const FilterJob &f, Mma8Job &j) { return mma8_job(f, 0, j); }
+
+cudaError_t launch_mma8_batch(const Mma8Job &rep, const Mma8Batch &b, int sm_count, cudaStream_t stream) {
+  if (b.tiles <= 0) return cudaSuccess;
+  return launch_fixed(rep, &b, sm_count, stream);
 }
 
 }  // namespace kcv

@@ -171,6 +171,20 @@ __device__ __forceinline__ uint32_t finish_sum(float acc, bool saturate) {
   else return bits;
 }
 
+// Bytes [sh, sh + 16) of the two blocks (0 <= sh < 16).
+__device__ __forceinline__ uint4 shift_blocks(const uint4 &u, const uint4 &v, int sh) {
+  const uint32_t w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+  const bool q1 = (sh & 4) != 0, q2 = (sh & 8) != 0;
+  uint32_t t[6], f[5];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) t[i] = q2 ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) f[i] = q1 ? t[i + 1] : t[i];
+  const int s8 = (sh & 3) * 8;
+  return make_uint4(__funnelshift_r(f[0], f[1], s8), __funnelshift_r(f[1], f[2], s8),
+                    __funnelshift_r(f[2], f[3], s8), __funnelshift_r(f[3], f[4], s8));
+}
+
 __device__ __forceinline__ void cp_async16_z(uint32_t dst, const void *src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
@@ -289,16 +303,7 @@ __device__ __forceinline__ void stage_pieces(const Mma8Job &j, uint8_t *raw, int
       for (int k = 0; k < kAhead; ++k) {
         uint8_t *d = raw + off + k * step * pitch;
         if (sh[k] >= 0) {
-          const uint32_t w[8] = {u[k].x, u[k].y, u[k].z, u[k].w, v[k].x, v[k].y, v[k].z, v[k].w};
-          const bool q1 = (sh[k] & 4) != 0, q2 = (sh[k] & 8) != 0;
-          uint32_t t[6], f[5], o[4];
-#pragma unroll
-          for (int i = 0; i < 6; ++i) t[i] = q2 ? w[i + 2] : w[i];
-#pragma unroll
-          for (int i = 0; i < 5; ++i) f[i] = q1 ? t[i + 1] : t[i];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) o[i] = __funnelshift_r(f[i], f[i + 1], (sh[k] & 3) * 8);
-          *reinterpret_cast<uint4 *>(d) = make_uint4(o[0], o[1], o[2], o[3]);
+          *reinterpret_cast<uint4 *>(d) = shift_blocks(u[k], v[k], sh[k]);
         } else if (row + k * step < rows) {
           const int y = map_index(y0 + row + k * step, j.h, j.border);
           if (y < 0) {
@@ -509,19 +514,51 @@ __device__ __forceinline__ void store_ragged(const Mma8Job &j, const uint8_t *st
     }
     return;
   }
-  // Words aligned in the destination, two rows at a time; bytes around them.
-  constexpr int kLanes = 4 * kPieces < 32 ? 4 * kPieces : 32, kRows = 32 / kLanes;
-  const int l = lane % kLanes;
-#pragma unroll 4
-  for (int row = lane / kLanes; row < rows; row += kRows) {
+  // Aligned 16-byte blocks of the destination, each from the two staged blocks
+  // around it; then the bytes before the first and after the last of them, one
+  // lane per row and end, as pieces of 1, 2, 4 and 8 bytes.
+  constexpr int kRows = 32 / kPieces;
+  const int p = lane % kPieces;
+#pragma unroll 2
+  for (int row = lane / kPieces; row < rows; row += kRows) {
     uint8_t *dd = d + static_cast<int64_t>(row) * j.dst_stride;
-    const uint8_t *sp = stg + row * kPitch;
-    const uint32_t *sw = reinterpret_cast<const uint32_t *>(sp);
-    const int hb = min(n, static_cast<int>(-reinterpret_cast<uintptr_t>(dd) & 3));
-    const int nw = (n - hb) >> 2, tb = n - hb - 4 * nw;
-    if (l < nw) *reinterpret_cast<uint32_t *>(dd + hb + 4 * l) = __funnelshift_r(sw[l], sw[l + 1], 8 * hb);
-    if (l < hb) dd[l] = sp[l];
-    if (l < tb) dd[n - tb + l] = sp[n - tb + l];
+    const int head = static_cast<int>(-reinterpret_cast<uintptr_t>(dd) & 15);  // bytes before the first block
+    if (head + 16 * p + 16 <= n) {
+      const uint8_t *sp = stg + row * kPitch + 16 * p;
+      const uint4 u = *reinterpret_cast<const uint4 *>(sp), v = *reinterpret_cast<const uint4 *>(sp + 16);
+      *reinterpret_cast<uint4 *>(dd + head + 16 * p) = shift_blocks(u, v, head);
+    }
+  }
+  const int row = lane >> 1;
+  if (row >= rows) return;
+  uint8_t *dd = d + static_cast<int64_t>(row) * j.dst_stride;
+  const uint8_t *sp = stg + row * kPitch;
+  const uint32_t *sw = reinterpret_cast<const uint32_t *>(sp);
+  const int head = static_cast<int>(-reinterpret_cast<uintptr_t>(dd) & 15);
+  if (head > n) {  // no whole block: a narrow last run
+    if ((lane & 1) == 0)
+      for (int i = 0; i < n; ++i) dd[i] = sp[i];
+    return;
+  }
+  const bool tail = (lane & 1) != 0;
+  const int from = tail ? head + (n - head) / 16 * 16 : 0;  // first byte of the end
+  const int c = tail ? n - from : head;                     // and its bytes
+  auto word = [&](int o) { return __funnelshift_r(sw[o >> 2], sw[(o >> 2) + 1], 8 * (o & 3)); };
+  if (c & 8) {
+    const int o = from + (tail ? 0 : c & 7);
+    *reinterpret_cast<uint2 *>(dd + o) = make_uint2(word(o), word(o + 4));
+  }
+  if (c & 4) {
+    const int o = from + (tail ? c & 8 : c & 3);
+    *reinterpret_cast<uint32_t *>(dd + o) = word(o);
+  }
+  if (c & 2) {
+    const int o = from + (tail ? c & 12 : c & 1);
+    *reinterpret_cast<uint16_t *>(dd + o) = static_cast<uint16_t>(word(o));
+  }
+  if (c & 1) {
+    const int o = from + (tail ? c & 14 : 0);
+    dd[o] = sp[o];
   }
 }
 
@@ -675,29 +712,26 @@ __device__ __forceinline__ void horizontal_pass(const Mma8Job &j, const Mma8Smem
   }
 }
 
-// The tiles blockIdx.x, + gridDim.x, ... of a job: a pipeline of steps (all
-// staged columns of a tile, or chunks of them where they do not fit), each
-// staged into one of two buffers while the step before it is computed.
+// Tiles first, first + stride, ... (`count` of them) of a job: a pipeline of
+// steps (all staged columns of a tile, or chunks of them where they do not
+// fit), each staged into one of two buffers while the step before it is
+// computed.  `taps` is cleared.
 template <int NK, int NB, int NA, int MT, int W, int EPI>
-__global__ void __launch_bounds__(kMma8Threads, NK != 1 ? 2 : 3)
-    mma8_kernel(const __grid_constant__ Mma8Job j) {
+__device__ __forceinline__ void mma8_tiles(const Mma8Job &j, Mma8Taps &taps, uint8_t *mem8, int first, int stride,
+                                           int count) {
   using G = Mma8Geo<NK, NB, MT, W>;
-  extern __shared__ __align__(16) uint8_t mem8[];
-  __shared__ __align__(4) Mma8Taps taps;
-  launch_dependents();
-  clear_taps(taps);
   Mma8Smem s;
   s.wa = reinterpret_cast<uint32_t *>(mem8);
-  s.wb = s.wa + j.nk * 64;
-  uint8_t *const raw0 = reinterpret_cast<uint8_t *>(s.wb + j.nb * 128);
+  s.wb = s.wa + (G::kFixed ? NK : j.nk) * 64;
+  uint8_t *const raw0 = reinterpret_cast<uint8_t *>(s.wb + (G::kFixed ? NB : j.nb) * 128);
   const int raw_bytes = max(G::raw_rows(j) * G::raw_pitch(j), mma8_out_bytes(mma8_run(MT, W)));
   s.raw = raw0;
   s.v = raw0 + 2 * raw_bytes;
   const int pitch = G::raw_pitch(j);
-  // The current tile, the distance to this CTA's next one, and the first
-  // column of the current step.
-  int ty = static_cast<int>(blockIdx.x) / j.tiles_x, tx = static_cast<int>(blockIdx.x) - ty * j.tiles_x;
-  const int dy = static_cast<int>(gridDim.x) / j.tiles_x, dx = static_cast<int>(gridDim.x) - dy * j.tiles_x;
+  // The current tile, the distance to the next one, and the first column of
+  // the current step.
+  int ty = first / j.tiles_x, tx = first - ty * j.tiles_x;
+  const int dy = stride / j.tiles_x, dx = stride - dy * j.tiles_x;
   int xb = tx * W - j.hp;
   auto stage = [&](uint8_t *raw) {
     const int xe = min(tx * W + W, j.wc) + j.rc;
@@ -706,11 +740,10 @@ __global__ void __launch_bounds__(kMma8Threads, NK != 1 ? 2 : 3)
   };
   __syncthreads();
   spread_taps(j, taps);
-  grid_dependency_wait();  // the source may be the previous call's output
   stage(s.raw);
   __syncthreads();
   build_weights(j, taps, s.wa, s.wb);
-  for (bool more = true; more;) {
+  while (count > 0) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     const int x0 = tx * W, y0 = ty * 16 * MT, cxb = xb;
@@ -730,17 +763,66 @@ __global__ void __launch_bounds__(kMma8Threads, NK != 1 ? 2 : 3)
       ty += dy;
       if (tx >= j.tiles_x) tx -= j.tiles_x, ++ty;
       xb = tx * W - j.hp;
-      more = ty < j.tiles_y;
+      --count;
     } else {
       xb += G::raw_cols(j);
     }
-    if (more) stage(next);
+    if (count > 0) stage(next);
     vertical_pass<NK, NB, MT, W, EPI>(j, s, x0, cxb, ncols);
     if (last) {
       __syncthreads();
       horizontal_pass<NK, NB, NA, MT, W, EPI>(j, s, x0, y0, we, rows);
     }
     s.raw = next;
+  }
+}
+
+template <int NK, int NB, int NA, int MT, int W, int EPI>
+__global__ void __launch_bounds__(kMma8Threads, NK != 1 ? 2 : 3) mma8_kernel(const __grid_constant__ Mma8Job j) {
+  extern __shared__ __align__(16) uint8_t mem8[];
+  __shared__ __align__(4) Mma8Taps taps;
+  launch_dependents();
+  clear_taps(taps);
+  grid_dependency_wait();  // the source may be the previous call's output
+  const int b = static_cast<int>(blockIdx.x), n = static_cast<int>(gridDim.x);
+  mma8_tiles<NK, NB, NA, MT, W, EPI>(j, taps, mem8, b, n, (j.tiles_x * j.tiles_y - b + n - 1) / n);
+}
+
+// Batch plans: one launch over a table of n jobs of one instantiation, of
+// which job k holds the tiles [ends[k - 1], ends[k]).  CTAs claim runs of
+// `chunk` tiles through *next (0 at launch).
+template <int NK, int NB, int NA, int MT, int W, int EPI>
+__global__ void __launch_bounds__(kMma8Threads, NK != 1 ? 2 : 3)
+    mma8_batch_kernel(const Mma8Job *__restrict__ jobs, const int *__restrict__ ends, int n, int chunk, int *next) {
+  extern __shared__ __align__(16) uint8_t mem8[];
+  __shared__ __align__(4) Mma8Taps taps;
+  __shared__ __align__(16) Mma8Job job;
+  __shared__ int claim;
+  const int total = ends[n - 1];
+  while (true) {
+    __syncthreads();  // the last run's shared memory is dead
+    if (threadIdx.x == 0) claim = atomicAdd(next, chunk);
+    __syncthreads();
+    int t = claim;
+    if (t >= total) return;
+    const int to = min(t + chunk, total);
+    while (t < to) {
+      int lo = 0, hi = n - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (ends[mid] > t) hi = mid;
+        else lo = mid + 1;
+      }
+      __syncthreads();
+      static_assert(sizeof(Mma8Job) % 4 == 0, "copied by words");
+      for (int i = threadIdx.x; i < static_cast<int>(sizeof(Mma8Job) / 4); i += kMma8Threads)
+        reinterpret_cast<uint32_t *>(&job)[i] = reinterpret_cast<const uint32_t *>(jobs + lo)[i];
+      clear_taps(taps);
+      __syncthreads();
+      const int from = lo > 0 ? ends[lo - 1] : 0, count = min(to, ends[lo]) - t;
+      mma8_tiles<NK, NB, NA, MT, W, EPI>(job, taps, mem8, t - from, 1, count);
+      t += count;
+    }
   }
 }
 

@@ -3,8 +3,9 @@
 
 namespace kcv {
 
-cudaError_t launch_mma8_3_3_3(const Mma8Job &j, int sm_count, cudaStream_t stream) {
-  return launch_mma8_tiled<3, 3, 3, kEpiRound>(j, sm_count, stream);
+cudaError_t launch_mma8_3_3_3(const Mma8Job &j, const Mma8Batch *batch, int sm_count,
+                             cudaStream_t stream) {
+  return launch_mma8_tiled<3, 3, 3, kEpiRound>(j, batch, sm_count, stream);
 }
 
 }  // namespace kcv
