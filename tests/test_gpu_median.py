@@ -117,3 +117,17 @@ def test_tall_narrow_images(case):
     w, h, c, k = case
     got, want, pad_ok = run("u8", w, h, c, k, 1, 21)
     assert pad_ok and np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", ["u8", "s16", "f32"])
+@pytest.mark.parametrize("k", [3, 5, 7])
+def test_block_edges(dtype, k):
+    """Widths and heights around a block's columns (128, or 64 for K = 7) and
+    rows (4, 8 and 16, by image size), one and several channels."""
+    ctx = kcv.Context.for_torch(0)
+    for n, (w, h, c) in enumerate([(127, 15, 1), (128, 16, 2), (129, 17, 3), (65, 9, 4), (63, 4 + k, 1),
+                                   (1290, 1027, 1), (1025, 801, 3), (2050, 515, 2)]):
+        got, want, pad_ok = run(dtype, w, h, c, k, (kcv.REPLICATE, kcv.REFLECT, kcv.WRAP, kcv.REVERSE)[n % 4],
+                                seed=100 * k + n, pad=n % 3, dpad=n % 2, ctx=ctx)
+        assert pad_ok and np.array_equal(got, want), (w, h, c)
+    ctx.close()
