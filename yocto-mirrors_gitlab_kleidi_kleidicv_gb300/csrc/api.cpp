@@ -545,35 +545,6 @@ kleidicv_error_t execute(kleidicv_gpu_context *ctx, Prepared &p) {
         ctx->launches += 1;
         return cuda_status(ctx, launch_sep16(p.fused, ctx->sm_count, ctx->stream));
       }
-      // A one-channel 16-bit call whose rows are not 16-byte aligned would take
-      // the tiled kernel; from 1 MiB up its source is first copied into a pool
-      // image with 16-byte rows so that the streaming kernel of sep16.cu takes
-      // it (3841x2160 u16: 34 us against 44 us).  Other modes gain nothing from
-      // the copy: the tiled kernel's loads and stores handle unaligned rows.
-      if (ctx->tune_threads <= 0) {
-        FilterJob probe = p.fused;
-        const long wcb = static_cast<long>(p.fused.width) * p.fused.channels * elem_size(p.fused.mode);
-        const size_t stride = (static_cast<size_t>(wcb) + 15) / 16 * 16;
-        probe.src = reinterpret_cast<const uint8_t *>(uintptr_t{256});  // any 16-byte aligned base
-        probe.src_stride = static_cast<int64_t>(stride);
-        if (static_cast<size_t>(wcb) * p.fused.height >= (size_t{1} << 20) && sep16_eligible(probe)) {
-          const size_t bytes = stride * p.fused.height;
-          uint8_t *realigned = static_cast<uint8_t *>(ctx_alloc(ctx, bytes));
-          if (realigned) {
-            cudaError_t e = launch_realign(p.fused.src, p.fused.src_stride, realigned, static_cast<int64_t>(stride),
-                                           wcb, p.fused.height, ctx->sm_count, ctx->stream);
-            if (e == cudaSuccess) {
-              p.fused.src = realigned;
-              p.fused.src_stride = static_cast<int64_t>(stride);
-              e = launch_sep16(p.fused, ctx->sm_count, ctx->stream);
-            }
-            ctx->launches += 2;
-            // Stream-ordered: the copy is released after the filter has read it.
-            ctx_free(ctx, realigned, bytes);
-            return cuda_status(ctx, e);
-          }
-        }
-      }
       if (ctx->tune_threads > 0) {
         TileShape t{ctx->tune_threads, ctx->tune_tile_rows, ctx->tune_stage_rows, ctx->tune_stages};
         apply_tile_shape(p.fused, t);

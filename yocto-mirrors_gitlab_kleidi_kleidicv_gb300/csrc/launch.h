@@ -57,9 +57,8 @@ cudaError_t launch_fused_batch(const FilterJob &rep, const BatchLaunch &b, int *
 int fused_batch_blocks_per_sm(const FilterJob &rep, const BatchLaunch &b);
 
 // separable_filter_2d u16 / s16 with 5x5 kernels on one channel
-// (csrc/sep16.cu).  sep16_eligible: the job is of that kind, its source rows
-// are 16-byte aligned, its destination allows 16-bit stores, and (s16) the
-// taps keep every sum exact in fp32.
+// (csrc/sep16.cu).  sep16_eligible: the job is of that kind, its rows are 2-byte
+// aligned, and (s16) the taps keep every sum exact in fp32.
 bool sep16_eligible(const FilterJob &job);
 cudaError_t launch_sep16(const FilterJob &job, int sm_count, cudaStream_t stream);
 
@@ -89,11 +88,6 @@ void pyr_entry(PyrEntry &e, const uint8_t *src, int64_t src_stride, uint8_t *dst
 // Resident warps of the pyramid kernel for `channels` on `sm_count` SMs (0 on
 // a CUDA failure).
 int pyramid_warps(int channels, int sm_count);
-
-// Copies `height` rows of `row_bytes` bytes (any source alignment) into
-// `dst`, whose base and stride are multiples of 16 (realign.cu).
-cudaError_t launch_realign(const uint8_t *src, int64_t src_stride, uint8_t *dst, int64_t dst_stride,
-                           long row_bytes, int height, int sm_count, cudaStream_t stream);
 
 // Generic per-element two-pass Gaussian (arbitrary sizes 11..255, and any
 // generated kernel whose weights do not sum to 256).  `scratch` holds the

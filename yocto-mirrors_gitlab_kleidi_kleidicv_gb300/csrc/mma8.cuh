@@ -171,20 +171,6 @@ __device__ __forceinline__ uint32_t finish_sum(float acc, bool saturate) {
   else return bits;
 }
 
-// Bytes [sh, sh + 16) of the two blocks (0 <= sh < 16).
-__device__ __forceinline__ uint4 shift_blocks(const uint4 &u, const uint4 &v, int sh) {
-  const uint32_t w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-  const bool q1 = (sh & 4) != 0, q2 = (sh & 8) != 0;
-  uint32_t t[6], f[5];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) t[i] = q2 ? w[i + 2] : w[i];
-#pragma unroll
-  for (int i = 0; i < 5; ++i) f[i] = q1 ? t[i + 1] : t[i];
-  const int s8 = (sh & 3) * 8;
-  return make_uint4(__funnelshift_r(f[0], f[1], s8), __funnelshift_r(f[1], f[2], s8),
-                    __funnelshift_r(f[2], f[3], s8), __funnelshift_r(f[3], f[4], s8));
-}
-
 __device__ __forceinline__ void cp_async16_z(uint32_t dst, const void *src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }

@@ -36,9 +36,12 @@
 // the band: the converted rows of the vertical window (five rows x 8 floats)
 // rotate through statically indexed register slots (the row loop is unrolled
 // by five), and each destination row costs one shared-memory load per lane.
-// The source rows must be 16-byte aligned (the host copies larger unaligned
-// sources into a 16-byte-row image first, and sends smaller ones to the
-// tiled kernel of sepfused.cuh).  This pass reads only the lanes whose 8 elements lie
+// Rows that are not 16-byte aligned are staged as the aligned blocks around
+// them (33 per strip); a lane then shifts its piece out of its block and the
+// next lane's, and stores go out as the aligned blocks that end in each
+// lane's piece, put together from its results and the previous lane's
+// (3841x2161 s16: 30 us with a realigning copy and a pool image before the
+// filter -> 20.6 us; 161x121 11.7 -> 5.5 us; aligned 3840x2160: 11.9 us).  This pass reads only the lanes whose 8 elements lie
 // inside the row, [0, wf) with wf = 8 * floor(w / 8), and stores only the
 // outputs whose five columns lie inside that span, x in [2, wf - 2).  The
 // other columns (x < 2 and x >= wf - 2) are edge elements, spread evenly over
@@ -64,8 +67,11 @@ constexpr int kWarps16 = kThreads16 / 32;
 constexpr int kLaneElems = 8;
 constexpr int kStripElems = kSep16Lanes * kLaneElems;
 constexpr int kStageRows = kSep16MaxBand + 4;          // source rows of a band
-constexpr int kWarpStageBytes = kStageRows * 32 * 16;  // 9728
-constexpr int kSmem16 = kWarps16 * kWarpStageBytes;    // 38912
+// 16-byte slots of a staged row: one per lane, and one block more where rows
+// are staged unaligned.
+constexpr int slots16(bool aligned) { return aligned ? 32 : 33; }
+constexpr int warp_stage16(bool aligned) { return kStageRows * slots16(aligned); }   // slots
+constexpr int smem16(bool aligned) { return kWarps16 * warp_stage16(aligned) * 16; }  // 38912, 40128
 constexpr int kGroups = (kStageRows + 4) / 5;          // copy groups of five rows: 4
 
 // No "memory" clobber: nothing reads the slot before cp_async_wait, which
@@ -208,11 +214,39 @@ __device__ __forceinline__ void edge_element16(const Sep16Job &j, int y, int x) 
   reinterpret_cast<uint16_t *>(j.dst + static_cast<int64_t>(y) * j.dst_stride)[x] = static_cast<uint16_t>(bits);
 }
 
-template <bool S16, bool SIMPLE>
-__device__ __forceinline__ void band_loop16(const Sep16Job &j, const uint4 *stage, int lane, int rows, uint8_t *d,
+// How a warp stores: whole aligned pieces; aligned pieces, and the pieces at
+// the row's ends by elements; pieces at any even address, those at the row's
+// ends by elements.
+enum Store16 { kStoreWhole, kStoreElements, kStoreShifted };
+
+template <bool S16, bool ALIGNED, int STORE>
+__device__ __forceinline__ void band_loop16(const Sep16Job &j, const uint4 *stage, int lane, int rows, int y0, uint8_t *d,
                                             long e0, int wf, bool outputs, bool full_store);
 
-template <bool S16>
+// Bytes by which row y of the source lies past a 16-byte boundary.
+__device__ __forceinline__ int row_shift(const Sep16Job &j, int y) {
+  return static_cast<int>(
+      (reinterpret_cast<uintptr_t>(j.src) + static_cast<uintptr_t>(static_cast<int64_t>(y) * j.src_stride)) & 15);
+}
+
+// The aligned block of row y that holds the first byte of the 8 elements at
+// e0, into `slot` (bytes past the image read as zero, none before it is read).
+__device__ __forceinline__ void stage_block16(const Sep16Job &j, uint4 *slot, int y, long e0) {
+  const uint8_t *a = j.src + static_cast<int64_t>(y) * j.src_stride + 2 * e0 - row_shift(j, y);
+  const int64_t left = j.src + static_cast<int64_t>(j.h - 1) * j.src_stride + 2 * static_cast<int64_t>(j.w) - a;
+  if (a >= j.src) {
+    const int n = left >= 16 ? 16 : left > 0 ? static_cast<int>(left) : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(slot))),
+                 "l"(n > 0 ? a : a - 16), "r"(n));
+  } else {
+    uint16_t *d = reinterpret_cast<uint16_t *>(slot);
+    for (int k = static_cast<int>(j.src - a) / 2; k < 8; ++k)
+      d[k] = 2 * k < left ? __ldg(reinterpret_cast<const uint16_t *>(a) + k) : uint16_t{0};
+  }
+}
+
+template <bool S16, bool ALIGNED>
 __device__ __forceinline__ void run_band16(const Sep16Job &j, uint4 *stage, int strip, int band, int lane) {
   const long e0 = static_cast<long>(strip) * kStripElems + kLaneElems * lane - kLaneElems;
   const int wf = full_span(j.w);
@@ -234,7 +268,44 @@ __device__ __forceinline__ void run_band16(const Sep16Job &j, uint4 *stage, int 
   // kGroups copy groups of five rows (rows [5g, 5g + 5); empty groups at the
   // end), so that the rows are filtered as their group lands.
   const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(stage + lane));
-  if (fast && y0 >= 2 && y1 + 2 <= j.h) {
+  if constexpr (!ALIGNED) {
+    // Every block that a lane inside the span reads: its own and the next.
+    const bool prev_fast = e0 - kLaneElems >= 0 && e0 <= wf;
+    int rr = 0;
+    if (y0 - 2 >= 1 && y1 + 2 <= j.h - 1 && j.src_stride >= 32) {
+      // Consecutive rows that are neither the image's first nor its last:
+      // every block lies in the image.
+      const bool own = fast || prev_fast, extra = lane == 31 && fast;
+      const uint8_t *g = j.src + static_cast<int64_t>(y0 - 2) * j.src_stride + 2 * e0;
+      uint32_t a = sbase;
+#pragma unroll
+      for (int grp = 0; grp < kGroups; ++grp) {
+#pragma unroll 1
+        for (; rr < min(nrows, 5 * grp + 5); ++rr, a += slots16(false) * 16, g += j.src_stride) {
+          const uint8_t *b = reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>(g) & ~uintptr_t{15});
+          if (own) cp_async16(a, b);
+          if (extra) cp_async16(a + 16, b + 16);
+        }
+        cp_async_commit();
+      }
+    } else
+#pragma unroll
+    for (int grp = 0; grp < kGroups; ++grp) {
+#pragma unroll 1
+      for (; rr < min(nrows, 5 * grp + 5); ++rr) {
+        const int y = map_index(y0 - 2 + rr, j.h, j.border);
+        uint4 *slot = stage + rr * slots16(false) + lane;
+        if (y < 0) {
+          slot[0] = make_uint4(bv2, bv2, bv2, bv2);
+          if (lane == 31) slot[1] = make_uint4(bv2, bv2, bv2, bv2);
+        } else {
+          if (fast || prev_fast) stage_block16(j, slot, y, e0);
+          if (lane == 31 && fast) stage_block16(j, slot + 1, y, e0 + kLaneElems);
+        }
+      }
+      cp_async_commit();
+    }
+  } else if (fast && y0 >= 2 && y1 + 2 <= j.h) {
     // Rows inside the image: consecutive.
     const uint8_t *g = j.src + static_cast<int64_t>(y0 - 2) * j.src_stride + 2 * e0;
     uint32_t a = sbase;
@@ -284,15 +355,67 @@ __device__ __forceinline__ void run_band16(const Sep16Job &j, uint4 *stage, int 
   }
 
   uint8_t *d = j.dst + static_cast<int64_t>(y0) * j.dst_stride + 2 * e0;
-  // The byte-store path only where some lane of the warp needs it.
   if (__all_sync(0xffffffffu, !outputs || full_store))
-    band_loop16<S16, true>(j, stage, lane, rows, d, e0, wf, outputs, full_store);
+    band_loop16<S16, ALIGNED, kStoreWhole>(j, stage, lane, rows, y0, d, e0, wf, outputs, full_store);
+  else if (((reinterpret_cast<uintptr_t>(j.dst) | static_cast<uintptr_t>(j.dst_stride)) & 15) != 0)
+    band_loop16<S16, ALIGNED, kStoreShifted>(j, stage, lane, rows, y0, d, e0, wf, outputs, full_store);
   else
-    band_loop16<S16, false>(j, stage, lane, rows, d, e0, wf, outputs, full_store);
+    band_loop16<S16, ALIGNED, kStoreElements>(j, stage, lane, rows, y0, d, e0, wf, outputs, full_store);
 }
 
-template <bool S16, bool SIMPLE>
-__device__ __forceinline__ void band_loop16(const Sep16Job &j, const uint4 *stage, int lane, int rows, uint8_t *d,
+// shift_blocks for a shift that is the same in every lane and even: branches
+// instead of selects.
+__device__ __forceinline__ uint4 shift_uniform(const uint4 &u, const uint4 &v, int sh) {
+  const int s8 = (sh & 3) * 8;
+  auto four = [&](uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e) {
+    return make_uint4(__funnelshift_r(a, b, s8), __funnelshift_r(b, c, s8), __funnelshift_r(c, d, s8),
+                      __funnelshift_r(d, e, s8));
+  };
+  switch (sh >> 2) {
+    case 0: return four(u.x, u.y, u.z, u.w, v.x);
+    case 1: return four(u.y, u.z, u.w, v.x, v.y);
+    case 2: return four(u.z, u.w, v.x, v.y, v.z);
+    default: return four(u.w, v.x, v.y, v.z, v.w);
+  }
+}
+
+// Stores a lane's 8 results at `d`, m = d % 16 bytes past a 16-byte boundary
+// (m even), as the aligned block that ends in them: its first m bytes are the
+// last of the previous lane's results `pr`.  For the first lane those are the
+// halo lane's (or those of the row's first piece), whose elements 2..7 are
+// exact, so only m = 14 makes it write its own 16 - m bytes by elements.  The
+// last lane's last m bytes are left to the next strip's first lane unless
+// `own_tail` or m = 14.
+__device__ __forceinline__ void store_shifted16(uint8_t *d, const uint4 &pr, const uint4 &r, bool outputs, bool first,
+                                                bool last, bool own_tail) {
+  const int m = static_cast<int>(reinterpret_cast<uintptr_t>(d) & 15);  // the same in every lane
+  if (m == 0) {
+    if (outputs) *reinterpret_cast<uint4 *>(d) = r;
+    return;
+  }
+  const uint4 block = shift_uniform(pr, r, 16 - m);
+  if (outputs && !(first && m == 14)) *reinterpret_cast<uint4 *>(d - m) = block;
+  if (m == 14 || own_tail) {
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+    uint16_t *d16 = reinterpret_cast<uint16_t *>(d);
+    const bool head = first && m == 14;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (2 * k < 16 - m ? head : last) d16[k] = static_cast<uint16_t>(w[k >> 1] >> (16 * (k & 1)));
+  }
+}
+
+// The elements [2, wf - 2) of a lane's 8 results.
+__device__ __forceinline__ void store_elements16(uint8_t *d, const uint4 &out, long e0, int wf) {
+  const uint32_t o[4] = {out.x, out.y, out.z, out.w};
+  uint16_t *d16 = reinterpret_cast<uint16_t *>(d);
+#pragma unroll
+  for (int k = 0; k < kLaneElems; ++k)
+    if (e0 + k >= 2 && e0 + k < wf - 2) d16[k] = static_cast<uint16_t>(o[k >> 1] >> (16 * (k & 1)));
+}
+
+template <bool S16, bool ALIGNED, int STORE>
+__device__ __forceinline__ void band_loop16(const Sep16Job &j, const uint4 *stage, int lane, int rows, int y0, uint8_t *d,
                                             long e0, int wf, bool outputs, bool full_store) {
   float2 kx[5], ky[5];
 #pragma unroll
@@ -300,11 +423,36 @@ __device__ __forceinline__ void band_loop16(const Sep16Job &j, const uint4 *stag
     kx[t] = make_float2(j.kx[t], j.kx[t]);
     ky[t] = make_float2(j.ky[t], j.ky[t]);
   }
+  const bool inner = y0 >= 2 && y0 + rows + 2 <= j.h;
+  const int shift0 = row_shift(j, y0 - 2), dshift = static_cast<int>(j.src_stride & 15);
+  // The lane's 8 elements of staged row rr.
+  auto piece = [&](int rr) {
+    const uint4 *slot = stage + rr * slots16(ALIGNED) + lane;
+    if constexpr (ALIGNED) {
+      return slot[0];
+    } else {
+      int sh = (shift0 + rr * dshift) & 15;  // consecutive rows
+      if (!inner) {
+        const int y = map_index(y0 - 2 + rr, j.h, j.border);
+        sh = y < 0 ? 0 : row_shift(j, y);
+      }
+      return shift_uniform(slot[0], slot[1], sh);
+    }
+  };
+  // Lanes whose whole piece is stored (kStoreShifted).
+  const bool inside = outputs && e0 >= 2 && e0 + kLaneElems <= wf - 2;
+  const unsigned in_lanes = __ballot_sync(0xffffffffu, inside);
+  const bool first = inside && (in_lanes & ((1u << lane) - 1)) == 0;
+  const bool last = inside && (in_lanes >> lane) == 1u;
+  const bool ends = __any_sync(0xffffffffu, outputs && !inside);
+  // The next strip stores by elements (its lanes reach the row's end).
+  const bool own_tail = e0 - kLaneElems * (lane - 1) + 2 * kStripElems > wf - 2;
   // Window slot k holds the converted source row rr with rr = k mod 5.
   float2 win[5][kLaneElems / 2];
   cp_async_wait<kGroups - 1>();  // group 0: rows 0 .. 4
+  if (!ALIGNED) __syncwarp();    // slots are read by two lanes
 #pragma unroll
-  for (int rr = 0; rr < 4; ++rr) to_float2<S16>(stage[rr * 32 + lane], win[rr]);
+  for (int rr = 0; rr < 4; ++rr) to_float2<S16>(piece(rr), win[rr]);
 #pragma unroll 1
   for (int base = 0; base < rows; base += 5) {
     // Destination rows base .. base + 4 read source rows up to base + 8:
@@ -314,31 +462,31 @@ __device__ __forceinline__ void band_loop16(const Sep16Job &j, const uint4 *stag
       case 1: cp_async_wait<kGroups - 3>(); break;
       default: cp_async_wait<0>(); break;
     }
+    if (!ALIGNED) __syncwarp();
     static_for<0, 5>([&](auto sc) {
       constexpr int S = decltype(sc)::value;
       constexpr int slot = (S + 4) % 5;  // receives source row rr = base + S + 4
       if (base + S >= rows) return;  // past the band (the loop ends here)
-      to_float2<S16>(stage[(base + S + 4) * 32 + lane], win[slot]);
+      to_float2<S16>(piece(base + S + 4), win[slot]);
       const uint4 out = filter_row<S16, S>(win, kx, ky);
-      if (SIMPLE) {
+      if constexpr (STORE == kStoreWhole) {
         if (outputs) *reinterpret_cast<uint4 *>(d) = out;
+      } else if constexpr (STORE == kStoreShifted) {
+        const uint4 prev = make_uint4(__shfl_up_sync(0xffffffffu, out.x, 1), __shfl_up_sync(0xffffffffu, out.y, 1),
+                                      __shfl_up_sync(0xffffffffu, out.z, 1), __shfl_up_sync(0xffffffffu, out.w, 1));
+        store_shifted16(d, prev, out, inside, first, last, own_tail);
+        if (ends && outputs && !inside) store_elements16(d, out, e0, wf);
       } else if (outputs) {
-        if (full_store) {
-          *reinterpret_cast<uint4 *>(d) = out;
-        } else {
-          const uint32_t o[4] = {out.x, out.y, out.z, out.w};
-          uint16_t *d16 = reinterpret_cast<uint16_t *>(d);
-#pragma unroll
-          for (int k = 0; k < kLaneElems; ++k)
-            if (e0 + k >= 2 && e0 + k < wf - 2) d16[k] = static_cast<uint16_t>(o[k >> 1] >> (16 * (k & 1)));
-        }
+        if (full_store) *reinterpret_cast<uint4 *>(d) = out;
+        else store_elements16(d, out, e0, wf);
       }
       d += j.dst_stride;
     });
   }
+  if (!ALIGNED) __syncwarp();  // the next item's copies may overwrite the slots
 }
 
-template <bool S16>
+template <bool S16, bool ALIGNED>
 __global__ void __launch_bounds__(kThreads16, 5) sep16_kernel(const __grid_constant__ Sep16Job j) {
   extern __shared__ __align__(16) uint4 stage16[];
   // The next call on the stream may start its CTAs as ours finish; it reads
@@ -346,7 +494,7 @@ __global__ void __launch_bounds__(kThreads16, 5) sep16_kernel(const __grid_const
   launch_dependents();
   grid_dependency_wait();  // the source may be the previous call's output
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint4 *stage = stage16 + warp * (kWarpStageBytes / 16);
+  uint4 *stage = stage16 + warp * warp_stage16(ALIGNED);
   // Items go round the CTAs first, so that every SM (the grid is whole
   // waves of resident CTAs) gets the same number.
   const int gw = warp * gridDim.x + blockIdx.x;
@@ -357,15 +505,15 @@ __global__ void __launch_bounds__(kThreads16, 5) sep16_kernel(const __grid_const
     // costlier strips at the row's ends.
     const int band = t / j.strips, q = t - band * j.strips;
     const int strip = static_cast<int>((q + 7L * band) % j.strips);
-    run_band16<S16>(j, stage, strip, band, lane);
+    run_band16<S16, ALIGNED>(j, stage, strip, band, lane);
   }
 }
 
-template <bool S16>
+template <bool S16, bool ALIGNED>
 cudaError_t launch16(Sep16Job &j, int sm_count, cudaStream_t stream) {
-  auto kern = sep16_kernel<S16>;
+  auto kern = sep16_kernel<S16, ALIGNED>;
   int occ = 0;
-  const cudaError_t err = resident_ctas_per_sm<sep16_kernel<S16>>(kThreads16, kSmem16, &occ);
+  const cudaError_t err = resident_ctas_per_sm<sep16_kernel<S16, ALIGNED>>(kThreads16, smem16(ALIGNED), &occ);
   if (err != cudaSuccess) return err;
   const long resident = static_cast<long>(occ) * std::max(sm_count, 1);
   const long slots = resident * kWarps16;
@@ -385,7 +533,7 @@ cudaError_t launch16(Sep16Job &j, int sm_count, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(kThreads16);
-  cfg.dynamicSmemBytes = kSmem16;
+  cfg.dynamicSmemBytes = smem16(ALIGNED);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -399,8 +547,8 @@ cudaError_t launch16(Sep16Job &j, int sm_count, cudaStream_t stream) {
 
 bool sep16_eligible(const FilterJob &f) {
   if ((f.mode != MODE_SEP_U16 && f.mode != MODE_SEP_S16) || f.ksize != 5 || f.channels != 1) return false;
-  // 16-byte copies of source rows; 16-bit destination stores.
-  if (((reinterpret_cast<uintptr_t>(f.src) | static_cast<uintptr_t>(f.src_stride)) & 15) != 0) return false;
+  // Whole elements.
+  if (((reinterpret_cast<uintptr_t>(f.src) | static_cast<uintptr_t>(f.src_stride)) & 1) != 0) return false;
   if (((reinterpret_cast<uintptr_t>(f.dst) | static_cast<uintptr_t>(f.dst_stride)) & 1) != 0) return false;
   // Item and edge indices in 32 bits.
   if (static_cast<long>(f.height) * (f.width / kStripElems + 1) >= (1L << 30) ||
@@ -429,7 +577,10 @@ cudaError_t launch_sep16(const FilterJob &f, int sm_count, cudaStream_t stream) 
     j.kx[t] = static_cast<float>(f.wx[t]);
     j.ky[t] = static_cast<float>(f.wy[t]);
   }
-  return f.mode == MODE_SEP_S16 ? launch16<true>(j, sm_count, stream) : launch16<false>(j, sm_count, stream);
+  const bool aligned = ((reinterpret_cast<uintptr_t>(f.src) | static_cast<uintptr_t>(f.src_stride)) & 15) == 0;
+  if (f.mode == MODE_SEP_S16)
+    return aligned ? launch16<true, true>(j, sm_count, stream) : launch16<true, false>(j, sm_count, stream);
+  return aligned ? launch16<false, true>(j, sm_count, stream) : launch16<false, false>(j, sm_count, stream);
 }
 
 }  // namespace kcv

@@ -91,6 +91,20 @@ __device__ __forceinline__ int map_index(int i, int n, int border) {
   return m < 0 ? 0 : (m >= n ? n - 1 : m);
 }
 
+// Bytes [sh, sh + 16) of the two blocks (0 <= sh < 16).
+__device__ __forceinline__ uint4 shift_blocks(const uint4 &u, const uint4 &v, int sh) {
+  const uint32_t w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+  const bool q1 = (sh & 4) != 0, q2 = (sh & 8) != 0;
+  uint32_t t[6], f[5];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) t[i] = q2 ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) f[i] = q1 ? t[i + 1] : t[i];
+  const int s8 = (sh & 3) * 8;
+  return make_uint4(__funnelshift_r(f[0], f[1], s8), __funnelshift_r(f[1], f[2], s8),
+                    __funnelshift_r(f[2], f[3], s8), __funnelshift_r(f[3], f[4], s8));
+}
+
 // Loads the in-image 16 bytes of a row at byte offset xb (0 <= xb, xb + 16 <=
 // row bytes) with 16-byte loads: directly when aligned, otherwise from the two
 // aligned blocks covering it when both lie inside the row.  Returns false when
@@ -105,16 +119,7 @@ __device__ __forceinline__ bool load_chunk_fast(const uint8_t *row, long xb, lon
   const uint8_t *a = reinterpret_cast<const uint8_t *>(pa & ~static_cast<uintptr_t>(15));
   if (a < row || a + 32 > row + wcb) return false;
   const uint4 u = ld_nc_v4(a), v = ld_nc_v4(a + 16);
-  const uint32_t w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-  const int sh = static_cast<int>(pa & 15), q = sh >> 2, s8 = (sh & 3) * 8;
-  uint32_t o[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint32_t lo = q == 0 ? w[k] : q == 1 ? w[k + 1] : q == 2 ? w[k + 2] : w[k + 3];
-    const uint32_t hi = q == 0 ? w[k + 1] : q == 1 ? w[k + 2] : q == 2 ? w[k + 3] : w[k + 4];
-    o[k] = __funnelshift_r(lo, hi, s8);
-  }
-  out = make_uint4(o[0], o[1], o[2], o[3]);
+  out = shift_blocks(u, v, static_cast<int>(pa & 15));
   return true;
 }
 
