@@ -516,15 +516,14 @@ kleidicv_error_t execute(kleidicv_gpu_context *ctx, Prepared &p) {
       if (p.fused.mode == MODE_BLURDOWN && ctx->tune_threads <= 0) {
         // One level: the tiled blur-and-downsample kernel of pyramid.cu.
         PyrLaunch L{};
-        pyr_entry(L.inline_entries[0], p.fused.src, p.fused.src_stride, p.fused.dst, p.fused.dst_stride,
+        PyrEntry entry;
+        pyr_entry(entry, p.fused.src, p.fused.src_stride, p.fused.dst, p.fused.dst_stride,
                   p.fused.width, p.fused.height, p.fused.channels, p.fused.border, p.fused.border_value,
                   pyramid_warps(p.fused.channels, ctx->sm_count));
-        L.phase_begin[0] = 0;
+        L.entries = &entry;
         L.phase_begin[1] = 1;
         L.phases = 1;
         L.channels = p.fused.channels;
-        L.barrier = reinterpret_cast<unsigned *>(ctx->d_err + 1);
-        L.err_flag = ctx->d_err;
         ctx->launches += 1;
         return cuda_status(ctx, launch_pyramid(L, ctx->sm_count, ctx->stream));
       }
@@ -603,10 +602,8 @@ kleidicv_error_t kleidicv_gpu_context_create(kleidicv_gpu_context_t **out, int d
   ctx->stream = static_cast<cudaStream_t>(stream);
   ctx->pool_limit = pool_limit_bytes ? pool_limit_bytes : (40ull << 30);
   ctx->sm_count = prop.multiProcessorCount;
-  // d_err[0]: the device error flag; d_err[1]: the pyramid kernel's grid
-  // barrier counter.
-  if (cudaMalloc(&ctx->d_err, 4 * sizeof(int)) != cudaSuccess ||
-      cudaMemset(ctx->d_err, 0, 4 * sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess ||
+      cudaMemset(ctx->d_err, 0, sizeof(int)) != cudaSuccess) {
     delete ctx;
     return KLEIDICV_GPU_ERROR_CUDA;
   }
@@ -852,22 +849,22 @@ kleidicv_error_t kleidicv_gpu_build_pyramid_u8(const uint8_t *src, size_t src_st
     }
     return KLEIDICV_OK;
   }
-  // Up to kPyrInline levels per launch, one phase per level.
-  for (size_t l0 = 0; l0 < levels; l0 += kPyrInline) {
-    const size_t n = std::min<size_t>(kPyrInline, levels - l0);
+  // One phase per level.
+  PyrEntry entries[64];
+  const int warps = pyramid_warps(static_cast<int>(channels), ctx->sm_count);
+  for (size_t l = 0; l < levels; ++l) {
+    const FilterJob &j = p[l].fused;
+    pyr_entry(entries[l], j.src, j.src_stride, j.dst, j.dst_stride, j.width, j.height, static_cast<int>(channels),
+              j.border, 0, warps);
+  }
+  for (size_t l0 = 0; l0 < levels; l0 += kPyrMaxPhases) {
+    const size_t n = std::min<size_t>(kPyrMaxPhases, levels - l0);
     PyrLaunch L{};
-    for (size_t k = 0; k < n; ++k) {
-      const FilterJob &j = p[l0 + k].fused;
-      pyr_entry(L.inline_entries[k], j.src, j.src_stride, j.dst, j.dst_stride, j.width, j.height,
-                static_cast<int>(channels), j.border, 0, pyramid_warps(static_cast<int>(channels), ctx->sm_count));
-      L.phase_begin[k] = static_cast<int32_t>(k);
-    }
-    L.phase_begin[n] = static_cast<int32_t>(n);
+    L.entries = entries + l0;
+    for (size_t k = 0; k <= n; ++k) L.phase_begin[k] = static_cast<int32_t>(k);
     L.phases = static_cast<int32_t>(n);
     L.channels = static_cast<int32_t>(channels);
-    L.barrier = reinterpret_cast<unsigned *>(ctx->d_err + 1);
-    L.err_flag = ctx->d_err;
-    ctx->launches += 1;
+    ctx->launches += n;
     e = cuda_status(ctx, launch_pyramid(L, ctx->sm_count, ctx->stream));
     if (e != KLEIDICV_OK) return e;
   }
@@ -904,7 +901,7 @@ kleidicv_error_t kleidicv_gpu_build_pyramids_u8(const kleidicv_gpu_pyramid_t *py
   kleidicv_error_t e = resolve_context(ctx);
   if (e != KLEIDICV_OK) return e;
   DeviceGuard guard(ctx->device);
-  // One launch per channel count: phase l holds level l + 1 of every image.
+  // Per channel count, phase l holds level l + 1 of every image.
   for (int c = 1; c <= static_cast<int>(kMaxChannels); ++c) {
     std::vector<PyrEntry> entries;
     PyrLaunch L{};
@@ -935,13 +932,10 @@ kleidicv_error_t kleidicv_gpu_build_pyramids_u8(const kleidicv_gpu_pyramid_t *py
     L.phase_begin[phases] = static_cast<int32_t>(entries.size());
     L.phases = static_cast<int32_t>(phases);
     L.channels = c;
-    L.barrier = reinterpret_cast<unsigned *>(ctx->d_err + 1);
-    L.err_flag = ctx->d_err;
+    L.entries = entries.data();
     const size_t bytes = entries.size() * sizeof(PyrEntry);
     PyrEntry *table = nullptr;
-    if (entries.size() <= static_cast<size_t>(kPyrInline)) {
-      std::copy(entries.begin(), entries.end(), L.inline_entries);
-    } else {
+    if (entries.size() > static_cast<size_t>(kPyrInline)) {
       table = static_cast<PyrEntry *>(ctx_alloc(ctx, bytes));
       if (!table) return KLEIDICV_ERROR_ALLOCATION;
       cudaError_t ce = upload_async(ctx, table, entries.data(), bytes);
@@ -949,9 +943,9 @@ kleidicv_error_t kleidicv_gpu_build_pyramids_u8(const kleidicv_gpu_pyramid_t *py
         ctx_free(ctx, table, bytes);
         return cuda_status(ctx, ce);
       }
-      L.entries = table;
+      L.table = table;
     }
-    ctx->launches += 1;
+    ctx->launches += phases;
     e = cuda_status(ctx, launch_pyramid(L, ctx->sm_count, ctx->stream));
     if (table) ctx_free(ctx, table, bytes);
     if (e != KLEIDICV_OK) return e;

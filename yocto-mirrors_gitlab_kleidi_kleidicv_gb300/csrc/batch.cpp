@@ -169,13 +169,11 @@ kleidicv_error_t enqueue(kleidicv_gpu_batch_plan *p, cudaStream_t s) {
   for (int c = 0; c < 4 && e == cudaSuccess; ++c) {
     if (p->pyr[c].empty()) continue;
     PyrLaunch L{};
-    L.entries = p->d_pyr[c];
-    L.phase_begin[0] = 0;
+    L.entries = p->pyr[c].data();
+    L.table = p->d_pyr[c];
     L.phase_begin[1] = static_cast<int32_t>(p->pyr[c].size());
     L.phases = 1;
     L.channels = c + 1;
-    L.barrier = reinterpret_cast<unsigned *>(ctx->d_err + 1);
-    L.err_flag = ctx->d_err;
     const size_t b = nb ? lane++ % nb : 0;
     used[b] = true;
     e = launch_pyramid(L, ctx->sm_count, nb ? p->branches[b] : s);

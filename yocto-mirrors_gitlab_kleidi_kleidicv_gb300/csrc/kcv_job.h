@@ -161,8 +161,7 @@ struct Mma8Job {
 // first its edge tasks (32 edge elements each), then (strip of 32 lanes of
 // source bytes, band of at most kPyrBandRows destination rows).  Entries are
 // grouped in phases: every entry of a phase depends only on earlier phases
-// (level l of every image is phase l - 1), and the kernel separates phases
-// with a grid-wide barrier.
+// (level l of every image is phase l - 1), and each phase is one launch.
 constexpr int kPyrBandRows = 8;
 constexpr int kPyrMaxPhases = 32;
 constexpr int kPyrInline = 8;  // entries carried in the launch parameters
@@ -180,13 +179,12 @@ struct PyrEntry {
 };
 
 struct PyrLaunch {
-  const PyrEntry *entries;  // device table, or nullptr: inline_entries
-  PyrEntry inline_entries[kPyrInline];
+  const PyrEntry *entries;  // on the host
+  const PyrEntry *table;    // the same on the device, or nullptr: at most
+                            // kPyrInline entries per phase, passed by value
   int32_t phase_begin[kPyrMaxPhases + 1];  // entries of phase p: [phase_begin[p], phase_begin[p+1])
   int32_t phases;
   int32_t channels;
-  unsigned *barrier;  // zero at launch when phases > 1
-  int *err_flag;      // set when a barrier wait hits its limit
 };
 
 // One entry of a batched work-list: tile (strip, band) of job `job`.

@@ -76,9 +76,8 @@ cudaError_t launch_gauss8_batch(int ksize, const Gauss8Job *table, int n, long i
                                 cudaStream_t stream);
 cudaError_t launch_gauss8(const FilterJob &job, int sm_count, cudaStream_t stream);
 
-// blur_and_downsample_u8 levels (csrc/pyramid.cu): L.phases phases of
-// entries, one launch (cooperative when there is more than one phase; the
-// barrier counter is cleared on the stream first).
+// blur_and_downsample_u8 levels (csrc/pyramid.cu): one launch per phase, in
+// order.
 cudaError_t launch_pyramid(const PyrLaunch &L, int sm_count, cudaStream_t stream);
 // Fills one level's entry: src (w x h x channels) -> dst ((w+1)/2 x (h+1)/2)
 // and its warp items (item_end = the entry's own count), its bands sized for

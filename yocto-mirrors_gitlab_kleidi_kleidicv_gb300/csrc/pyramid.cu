@@ -33,11 +33,12 @@
 // edge tasks of the same phase, scheduled first: one lane per (row, element),
 // its 25 border-mapped source bytes loaded independently.
 //
-// A pyramid is one launch: each level of each image is a phase, and phases
-// are separated by a grid-wide barrier (every CTA resident: cooperative
-// launch).  Level l + 1 reads level l right after it was written, mostly from
-// L2, through copies and loads that bypass L1.  Every barrier wait is bounded;
-// on expiry the kernel sets the error flag and returns.
+// A pyramid is one launch per level (level l of all images of a batched call
+// together), each started early by programmatic dependent launch: its CTAs
+// are resident when the level before completes.  One cooperative launch with
+// grid-wide barriers between the levels cost about 10 us for the launch and
+// the barrier's reset and 3 to 6 us per barrier: 8192x8192x1, five levels,
+// 64.5 -> PYA us; 256x256x1, four levels, 16.3 -> PYB us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -55,8 +56,7 @@ constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
 constexpr int kStageRows = 2 * kPyrBandRows + 3;
 constexpr int kGroups = (kStageRows + 4) / 5;  // copy groups of five rows: 4
-constexpr uint64_t kBarrierLimitNs = 2000000000ull;
-constexpr int kPyrSearchEntries = 512;  // phases with more entries search in global memory
+constexpr int kPyrSearchEntries = 512;  // launches of more entries search in global memory
 
 // Lane geometry for C channels.
 template <int C>
@@ -96,18 +96,7 @@ __host__ __device__ constexpr uint32_t tap_word(int c, int j, int q) {
   return w;
 }
 
-template <bool FRESH>
-__device__ __forceinline__ uint32_t ld8(const uint8_t *p) {
-  uint16_t v;
-  if (FRESH)
-    asm("ld.global.cg.u8 %0, [%1];" : "=h"(v) : "l"(p));
-  else
-    asm("ld.global.nc.u8 %0, [%1];" : "=h"(v) : "l"(p));
-  return v;
-}
-
-// cp.async.cg goes through L2 only: safe for a source written earlier in the
-// same launch.  No "memory" clobber: nothing reads the slot before the wait.
+// No "memory" clobber: nothing reads the slot before the wait.
 __device__ __forceinline__ void cp_async16p(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
 }
@@ -126,37 +115,6 @@ __device__ __forceinline__ void wait_groups(int pending) {
     default: cp_async_wait_p<3>(); break;
   }
   __syncwarp();
-}
-
-__device__ __forceinline__ uint32_t ld_acquire_u32(const unsigned *p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Grid-wide barrier number `epoch` (1, 2, ...): every CTA adds one to the
-// counter and waits until all gridDim.x CTAs have, at most kBarrierLimitNs.
-__device__ bool grid_barrier(unsigned *count, unsigned epoch, int *err_flag) {
-  __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();  // this CTA's outputs before its arrival
-    atomicAdd(count, 1u);
-    const unsigned target = epoch * gridDim.x;
-    const uint64_t start = global_timer_ns();
-    int good = 1;
-    while (ld_acquire_u32(count) < target) {
-      if (global_timer_ns() - start > kBarrierLimitNs) {
-        atomicOr(err_flag, 1);
-        good = 0;
-        break;
-      }
-      __nanosleep(100);
-    }
-    ok = good;
-  }
-  __syncthreads();
-  return ok != 0;
 }
 
 // Horizontal sums of the lane's tap window t (NT source words) for its OUT
@@ -244,7 +202,7 @@ __host__ __device__ inline bool rows_aligned(const uint8_t *src, int64_t stride)
 
 // One band of one strip of one entry (ALIGNED: 16-byte aligned base and
 // stride).
-template <int C, bool FRESH, bool ALIGNED>
+template <int C, bool ALIGNED>
 __device__ __forceinline__ void run_band(const PyrEntry &e, uint8_t *stage, int strip, int band, int lane) {
   using G = LaneGeo<C>;
   const long wc = static_cast<long>(e.w) * C;
@@ -370,7 +328,7 @@ __host__ __device__ inline EdgeSplit edge_split(int w, int ow, int c, bool align
 
 // Edge task `task` of entry e: destination element (Y, X, ch) of an edge
 // pixel.
-template <int C, bool FRESH>
+template <int C>
 __device__ __forceinline__ void edge_task(const PyrEntry &e, int task) {
   const EdgeSplit sp = edge_split(e.w, e.ow, C, rows_aligned(e.src, e.src_stride));
   const int per_row = sp.per_row;
@@ -392,7 +350,7 @@ __device__ __forceinline__ void edge_task(const PyrEntry &e, int task) {
 #pragma unroll
   for (int r = 0; r < 5; ++r)
 #pragma unroll
-    for (int c = 0; c < 5; ++c) v[r][c] = (rows[r] && cols[c] >= 0) ? ld8<FRESH>(rows[r] + cols[c]) : bv;
+    for (int c = 0; c < 5; ++c) v[r][c] = (rows[r] && cols[c] >= 0) ? __ldg(rows[r] + cols[c]) : bv;
   const uint32_t wt[5] = {1, 4, 6, 4, 1};
   uint32_t sum = 128;
 #pragma unroll
@@ -403,10 +361,10 @@ __device__ __forceinline__ void edge_task(const PyrEntry &e, int task) {
   e.dst[static_cast<int64_t>(Y) * e.dst_stride + static_cast<long>(X) * C + ch] = static_cast<uint8_t>(sum >> 8);
 }
 
-template <int C, bool FRESH>
+template <int C>
 __device__ __forceinline__ void run_item(const PyrEntry &en, uint8_t *stage, int local, int lane) {
   if (local < en.edge_items) {
-    edge_task<C, FRESH>(en, local * 32 + lane);
+    edge_task<C>(en, local * 32 + lane);
   } else {
     // Strips rotate by 7 per band: a warp's items do not all land on the
     // strips at the row's ends.
@@ -414,50 +372,48 @@ __device__ __forceinline__ void run_item(const PyrEntry &en, uint8_t *stage, int
     const int band = m / en.strips, q = m - band * en.strips;
     const int strip = static_cast<int>((q + 7L * band) % en.strips);
     if (rows_aligned(en.src, en.src_stride))
-      run_band<C, FRESH, true>(en, stage, strip, band, lane);
+      run_band<C, true>(en, stage, strip, band, lane);
     else
-      run_band<C, FRESH, false>(en, stage, strip, band, lane);
+      run_band<C, false>(en, stage, strip, band, lane);
   }
 }
 
+// One launch: n entries, in a device table or in the parameters.
+struct PyrPhase {
+  const PyrEntry *entries;  // nullptr: inline_entries
+  PyrEntry inline_entries[kPyrInline];
+  int32_t n;
+};
+
 template <int C>
-__global__ void __launch_bounds__(kThreads) pyramid_kernel(const __grid_constant__ PyrLaunch L) {
+__global__ void __launch_bounds__(kThreads) pyramid_kernel(const __grid_constant__ PyrPhase L) {
   extern __shared__ __align__(16) uint8_t pyr_stage[];
   launch_dependents();
-  grid_dependency_wait();  // the source may be the previous call's output
+  grid_dependency_wait();  // the source may be the previous launch's output
   const PyrEntry *E = L.entries ? L.entries : L.inline_entries;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint8_t *stage = pyr_stage + warp * LaneGeo<C>::WARP_STAGE;
   // Items go round the CTAs first, so that every SM gets the same number.
   const int gwarp = warp * gridDim.x + blockIdx.x;
   const int nwarps = gridDim.x * kWarps;
-  // The phase's item boundaries, for the entry search (a table in global
+  // The entries' item boundaries, for the entry search (a table in global
   // memory would make every search a chain of dependent loads).
   __shared__ int ends[kPyrSearchEntries];
-  for (int ph = 0; ph < L.phases; ++ph) {
-    if (ph > 0 && !grid_barrier(L.barrier, static_cast<unsigned>(ph), L.err_flag)) return;
-    const int e0 = L.phase_begin[ph], e1 = L.phase_begin[ph + 1];
-    const bool cached = e1 - e0 <= kPyrSearchEntries;
-    __syncthreads();  // the previous phase's readers of ends[] are done
-    if (cached)
-      for (int k = threadIdx.x; k < e1 - e0; k += blockDim.x) ends[k] = E[e0 + k].item_end;
-    __syncthreads();
-    const int total = E[e1 - 1].item_end;
-    for (int t = gwarp; t < total; t += nwarps) {
-      // The entry holding item t: the first with item_end > t.
-      int lo = e0, hi = e1 - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) / 2;
-        if ((cached ? ends[mid - e0] : E[mid].item_end) > t) hi = mid;
-        else lo = mid + 1;
-      }
-      const PyrEntry en = E[lo];  // one round of loads, then registers
-      const int local = t - (lo > e0 ? (cached ? ends[lo - 1 - e0] : E[lo - 1].item_end) : 0);
-      if (ph == 0)
-        run_item<C, false>(en, stage, local, lane);
-      else
-        run_item<C, true>(en, stage, local, lane);
+  const bool cached = L.n <= kPyrSearchEntries;
+  if (cached)
+    for (int k = threadIdx.x; k < L.n; k += blockDim.x) ends[k] = E[k].item_end;
+  __syncthreads();
+  const int total = E[L.n - 1].item_end;
+  for (int t = gwarp; t < total; t += nwarps) {
+    // The entry holding item t: the first with item_end > t.
+    int lo = 0, hi = L.n - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi) / 2;
+      if ((cached ? ends[mid] : E[mid].item_end) > t) hi = mid;
+      else lo = mid + 1;
     }
+    const PyrEntry en = E[lo];  // one round of loads, then registers
+    run_item<C>(en, stage, t - (lo > 0 ? (cached ? ends[lo - 1] : E[lo - 1].item_end) : 0), lane);
   }
 }
 
@@ -470,35 +426,29 @@ int warps_c(int sm_count) {
 
 template <int C>
 cudaError_t launch_c(const PyrLaunch &L, int sm_count, cudaStream_t stream) {
-  auto kern = pyramid_kernel<C>;
   const int warps = warps_c<C>(sm_count);
   if (warps == 0) return cudaErrorInvalidValue;
-  const PyrEntry *E = L.entries ? nullptr : L.inline_entries;
-  long most = 1;
-  if (E) {
-    for (int ph = 0; ph < L.phases; ++ph)
-      most = std::max<long>(most, E[L.phase_begin[ph + 1] - 1].item_end);
-  } else {
-    most = 1L << 40;  // device table: the caller sized the phases
-  }
-  const int grid = static_cast<int>(std::max(1L, std::min<long>(warps / kWarps, (most + kWarps - 1) / kWarps)));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem_bytes<C>();
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  if (L.phases > 1) {
-    // Grid-wide barriers need every CTA resident.
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-  } else {
+  for (int ph = 0; ph < L.phases; ++ph) {
+    const int e0 = L.phase_begin[ph], e1 = L.phase_begin[ph + 1];
+    PyrPhase p{};
+    p.n = e1 - e0;
+    if (L.table) p.entries = L.table + e0;
+    else std::copy(L.entries + e0, L.entries + e1, p.inline_entries);
+    const long items = L.entries[e1 - 1].item_end;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(std::max(1L, std::min<long>(warps / kWarps, (items + kWarps - 1) / kWarps))));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem_bytes<C>();
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, pyramid_kernel<C>, p);
+    if (e != cudaSuccess) return e;
   }
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, L);
+  return cudaSuccess;
 }
 
 }  // namespace
@@ -514,10 +464,6 @@ int pyramid_warps(int channels, int sm_count) {
 }
 
 cudaError_t launch_pyramid(const PyrLaunch &L, int sm_count, cudaStream_t stream) {
-  if (L.phases > 1) {
-    const cudaError_t e = cudaMemsetAsync(L.barrier, 0, sizeof(unsigned), stream);
-    if (e != cudaSuccess) return e;
-  }
   switch (L.channels) {
     case 1: return launch_c<1>(L, sm_count, stream);
     case 2: return launch_c<2>(L, sm_count, stream);
