@@ -372,7 +372,7 @@ kleidicv_error_t kleidicv_gpu_batch_submit(const kleidicv_gpu_request_t *request
                                            kleidicv_error_t *statuses,
                                            kleidicv_gpu_context_t *ctx);
 
-/* Many image pyramids in one launch per channel count (no reference
+/* Many image pyramids in one launch per level and channel count (no reference
  * counterpart: the reference builds every pyramid level by level).  Each
  * entry is validated like kleidicv_gpu_build_pyramid_u8 (statuses[i] is its
  * result, statuses may be NULL); valid entries are computed, level l of every

@@ -162,7 +162,7 @@ struct Mma8Job {
 // source bytes, band of at most kPyrBandRows destination rows).  Entries are
 // grouped in phases: every entry of a phase depends only on earlier phases
 // (level l of every image is phase l - 1), and each phase is one launch.
-constexpr int kPyrBandRows = 8;
+constexpr int kPyrBandRows = 32;
 constexpr int kPyrMaxPhases = 32;
 constexpr int kPyrInline = 8;  // entries carried in the launch parameters
 

@@ -9,10 +9,11 @@
 //
 // A warp owns a strip of 32 lanes x B source bytes (B = 16, or 24 for three
 // channels) and a band of at most kPyrBandRows destination rows:
-//  * it requests the band's 2 * rows + 3 source rows at once: the strip's
-//    bytes plus a 16-byte chunk on either side, as 16-byte cp.async chunks
-//    spread over the lanes, into the warp's shared-memory rows, in copy
-//    groups of five rows that are filtered as they land;
+//  * it keeps four copy groups of four source rows in flight down the band:
+//    the strip's bytes plus a 16-byte chunk on either side, as 16-byte cp.async
+//    chunks spread over the lanes, into a ring of the warp's shared-memory
+//    rows, so that copies and arithmetic overlap (bands of 8 rows whose copies
+//    were all issued first: 8192x8192x1 23.8 us, now 18.6 us);
 //  * horizontal pass: each lane reads its tap window (its B bytes and the
 //    words around them) from the staged row.  For one to three channels every
 //    destination element is a chain of dp4a over the words its five taps fall
@@ -38,7 +39,7 @@
 // are resident when the level before completes.  One cooperative launch with
 // grid-wide barriers between the levels cost about 10 us for the launch and
 // the barrier's reset and 3 to 6 us per barrier: 8192x8192x1, five levels,
-// 64.5 -> PYA us; 256x256x1, four levels, 16.3 -> PYB us.
+// 64.5 -> 44.9 us; 256x256x1, four levels, 16.3 -> 11.2 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -54,8 +55,8 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
-constexpr int kStageRows = 2 * kPyrBandRows + 3;
-constexpr int kGroups = (kStageRows + 4) / 5;  // copy groups of five rows: 4
+constexpr int kGroupRows = 4, kRingGroups = 4;  // staged rows: a ring of copy groups
+constexpr int kStageRows = kGroupRows * kRingGroups;
 constexpr int kPyrSearchEntries = 512;  // launches of more entries search in global memory
 
 // Lane geometry for C channels.
@@ -105,18 +106,6 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait_p() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-// Waits until at most `pending` copy groups are outstanding, then makes the
-// warp's copies visible to all its lanes.
-__device__ __forceinline__ void wait_groups(int pending) {
-  switch (pending) {
-    case 0: cp_async_wait_p<0>(); break;
-    case 1: cp_async_wait_p<1>(); break;
-    case 2: cp_async_wait_p<2>(); break;
-    default: cp_async_wait_p<3>(); break;
-  }
-  __syncwarp();
-}
-
 // Horizontal sums of the lane's tap window t (NT source words) for its OUT
 // destination elements, as NH packed 16-bit pairs (sums <= 4080).
 template <int C>
@@ -213,44 +202,56 @@ __device__ __forceinline__ void run_band(const PyrEntry &e, uint8_t *stage, int 
 
   const int rows = e.band_q + (band < e.band_r ? 1 : 0);
   const int Y0 = band * e.band_q + min(band, e.band_r);
-  const int nrows = 2 * rows + 3;  // source rows 2 Y0 - 2 .. 2 Y1
+  const int nrows = 2 * rows + 3;  // source rows y0 .. y0 + nrows - 1
+  const int y0 = 2 * Y0 - 2;
 
-  // Copies: row rr of the stage holds source row 2 Y0 - 2 + rr from row byte
-  // base - mis (mis: the row start's misalignment, 0 when aligned and for a
-  // constant-border row); each lane copies chunks lane and lane + 32 of it,
-  // the aligned blocks wholly inside the row.  The misalignments are kept as
-  // 4-bit fields for the reads.
-  const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(stage));
-  uint64_t mis_lo = 0;  // rows 0 .. 15
-  uint32_t mis_hi = 0;  // rows 16 .. 18
-  int rr = 0;
-#pragma unroll
-  for (int grp = 0; grp < kGroups; ++grp) {
+  // Copy group k: staged rows 4k .. 4k + 3, into ring group k % 4.  Staged row
+  // rr holds source row y0 + rr from row byte base - mis (mis: the row start's
+  // misalignment, 0 when aligned and for a constant-border row); each lane
+  // copies chunks lane and lane + 32 of it, the aligned blocks wholly inside
+  // the row.  The ring's misalignments are kept as 4-bit fields for the reads.
+  const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(stage)) + 16 * lane;
+  const long x = base + 16L * lane;  // row byte of the lane's first chunk, + mis
+  const bool second = lane + 32 < G::CHUNKS;
+  const bool inner = y0 >= 0 && y0 + nrows <= e.h;
+  uint64_t mis_ring = 0;
+  auto copy_group = [&](int k) {
+    const int sh = 16 * (k % kRingGroups);
+    if constexpr (!ALIGNED) mis_ring &= ~(0xFFFFull << sh);
+    const int last = min(nrows, kGroupRows * k + kGroupRows);
+    uint32_t a = sbase + (k % kRingGroups) * kGroupRows * G::ROW;
+    if (ALIGNED && inner) {
+      const uint8_t *g = e.src + static_cast<int64_t>(y0 + kGroupRows * k) * e.src_stride + x;
+      const bool c0 = x >= 0 && x + 16 <= wc, c1 = second && x + 528 <= wc;
 #pragma unroll 1
-    for (; rr < min(nrows, 5 * grp + 5); ++rr) {
-      const int y = map_index(2 * Y0 - 2 + rr, e.h, e.border);
-      const uint8_t *srow = y < 0 ? e.src : e.src + static_cast<int64_t>(y) * e.src_stride;
-      const int mis = (ALIGNED || y < 0) ? 0 : static_cast<int>(reinterpret_cast<uintptr_t>(srow) & 15);
-      if constexpr (!ALIGNED) {
-        if (rr < 16) mis_lo |= static_cast<uint64_t>(mis) << (4 * rr);
-        else mis_hi |= static_cast<uint32_t>(mis) << (4 * (rr - 16));
+      for (int rr = kGroupRows * k; rr < last; ++rr, a += G::ROW, g += e.src_stride) {
+        if (c0) cp_async16p(a, g);
+        if (c1) cp_async16p(a + 512, g + 512);
       }
-#pragma unroll
-      for (int k = lane; k < G::CHUNKS; k += 32) {
-        const long x = base + 16L * k - mis;
+    } else {
+#pragma unroll 1
+      for (int rr = kGroupRows * k; rr < last; ++rr, a += G::ROW) {
+        const int y = map_index(y0 + rr, e.h, e.border);
         if (y < 0) {
-          *reinterpret_cast<uint4 *>(stage + rr * G::ROW + 16 * k) = make_uint4(bv4, bv4, bv4, bv4);
-        } else if (x >= 0 && x + 16 <= wc) {
-          cp_async16p(sbase + rr * G::ROW + 16 * k, srow + x);
+          uint4 *d = reinterpret_cast<uint4 *>(stage + (rr % kStageRows) * G::ROW) + lane;
+          d[0] = make_uint4(bv4, bv4, bv4, bv4);
+          if (second) d[32] = make_uint4(bv4, bv4, bv4, bv4);
+          continue;
         }
+        const uint8_t *srow = e.src + static_cast<int64_t>(y) * e.src_stride;
+        const int mis = ALIGNED ? 0 : static_cast<int>(reinterpret_cast<uintptr_t>(srow) & 15);
+        if constexpr (!ALIGNED) mis_ring |= static_cast<uint64_t>(mis) << (sh + 4 * (rr % kGroupRows));
+        if (x - mis >= 0 && x - mis + 16 <= wc) cp_async16p(a, srow + x - mis);
+        if (second && x - mis + 512 >= 0 && x - mis + 528 <= wc) cp_async16p(a + 512, srow + x - mis + 512);
       }
     }
     cp_async_commit_p();
-  }
-  auto mis_of = [&](int row) -> int {
-    if constexpr (ALIGNED) return 0;
-    return row < 16 ? static_cast<int>((mis_lo >> (4 * row)) & 15) : static_cast<int>((mis_hi >> (4 * (row - 16))) & 15);
   };
+#pragma unroll 1
+  for (int k = 0; k < kRingGroups; ++k) copy_group(k);
+  // Row i of ring group q.
+  auto row_at = [&](int q, int i) { return stage + (q * kGroupRows + i) * G::ROW; };
+  auto mis_at = [&](int q, int i) { return ALIGNED ? 0 : static_cast<int>(mis_ring >> (16 * q + 4 * i)) & 15; };
 
   // Stored: destination elements of pixels [xl, xr].
   const Interior in = interior(e.w, C, ALIGNED);
@@ -262,19 +263,16 @@ __device__ __forceinline__ void run_band(const PyrEntry &e, uint8_t *stage, int 
       oe >= olo && oe + G::OUT <= ohi &&
       ((reinterpret_cast<uintptr_t>(e.dst) | static_cast<uintptr_t>(e.dst_stride)) & smask) == 0;
 
-  uint32_t a[G::NH], b[G::NH], c[G::NH];
-  wait_groups(kGroups - 1);  // group 0: rows 0 .. 4
-  hsums<C, ALIGNED>(stage, off, mis_of(0), a);
-  hsums<C, ALIGNED>(stage + G::ROW, off, mis_of(1), b);
-  hsums<C, ALIGNED>(stage + 2 * G::ROW, off, mis_of(2), c);
+  uint32_t a[G::NH], b[G::NH], c[G::NH];  // sums of source rows 2r, 2r + 1, 2r + 2 of destination row r
+  cp_async_wait_p<kRingGroups - 1>();     // group 0
+  __syncwarp();
+  hsums<C, ALIGNED>(row_at(0, 0), off, mis_at(0, 0), a);
+  hsums<C, ALIGNED>(row_at(0, 1), off, mis_at(0, 1), b);
+  hsums<C, ALIGNED>(row_at(0, 2), off, mis_at(0, 2), c);
   uint8_t *drow = e.dst + static_cast<int64_t>(Y0) * e.dst_stride + oe;
-#pragma unroll 1
-  for (int r = 0; r < rows; ++r) {
-    // Destination row r reads stage rows 2r + 3 and 2r + 4: group (2r + 4) / 5.
-    wait_groups(max(0, kGroups - 1 - (2 * r + 4) / 5));
-    uint32_t d[G::NH], ee[G::NH];
-    hsums<C, ALIGNED>(stage + (2 * r + 3) * G::ROW, off, mis_of(2 * r + 3), d);
-    hsums<C, ALIGNED>(stage + (2 * r + 4) * G::ROW, off, mis_of(2 * r + 4), ee);
+  // The next destination row from the sums a, b, c and those of its last two
+  // source rows.
+  auto emit = [&](const uint32_t(&d)[G::NH], const uint32_t(&ee)[G::NH]) {
     uint32_t s[G::NH];
 #pragma unroll
     for (int k = 0; k < G::NH; ++k) s[k] = a[k] + ee[k] + 0x00800080u + 4u * (b[k] + d[k]) + 6u * c[k];
@@ -306,9 +304,29 @@ __device__ __forceinline__ void run_band(const PyrEntry &e, uint8_t *stage, int 
       b[k] = d[k];
       c[k] = ee[k];
     }
+  };
+  // Destination rows 2m and 2m + 1 read staged rows 4m + 3 .. 4m + 6: the last
+  // of group m, whose slots then take group m + 4, and three of group m + 1.
+#pragma unroll 1
+  for (int m = 0; 2 * m < rows; ++m) {
+    cp_async_wait_p<kRingGroups - 2>();  // groups up to m + 1 of m + 4
+    __syncwarp();
+    const int q0 = m % kRingGroups, q1 = (m + 1) % kRingGroups;
+    uint32_t d[G::NH], ee[G::NH];
+    hsums<C, ALIGNED>(row_at(q0, 3), off, mis_at(q0, 3), d);
+    hsums<C, ALIGNED>(row_at(q1, 0), off, mis_at(q1, 0), ee);
+    __syncwarp();  // every lane has read group m
+    copy_group(m + kRingGroups);
+    emit(d, ee);
+    if (2 * m + 1 < rows) {
+      hsums<C, ALIGNED>(row_at(q1, 1), off, mis_at(q1, 1), d);
+      hsums<C, ALIGNED>(row_at(q1, 2), off, mis_at(q1, 2), ee);
+      emit(d, ee);
+    }
   }
   // The stage is rewritten by the warp's next item only after every lane
-  // has read it.
+  // has read it and no copy is outstanding.
+  cp_async_wait_p<0>();
   __syncwarp();
 }
 
@@ -492,8 +510,8 @@ void pyr_entry(PyrEntry &e, const uint8_t *src, int64_t src_stride, uint8_t *dst
   const long strip_out = 32L * (channels == 3 ? 12 : 8);
   const long owc = static_cast<long>(e.ow) * channels;
   e.strips = sp.xs > sp.xl ? static_cast<int32_t>((owc + strip_out - 1) / strip_out) : 0;
-  // Bands of at most kPyrBandRows rows, as many as give every warp the same
-  // number of items.
+  // Bands of at most kPyrBandRows rows (so that a batch of uneven images stays
+  // balanced), as many as give every warp the same number of items.
   long bands = 0;
   if (e.strips > 0) {
     const long min_bands = (e.oh + kPyrBandRows - 1) / kPyrBandRows;
