@@ -372,7 +372,7 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
     const int share = std::max(1, gauss8_batch_warps(3 + 2 * k, ctx->sm_count) / static_cast<int>(v.size()));
     int32_t items = 0;
     for (Gauss8Job &g : v) {
-      gauss8_size_for_share(g, share);
+      gauss8_size_for_share(g, 3 + 2 * k, share);
       items += g.strips * g.bands;
       g.item_end = items;
     }

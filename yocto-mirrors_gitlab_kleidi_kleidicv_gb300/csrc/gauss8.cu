@@ -13,11 +13,14 @@
 //
 // A warp owns a strip of 32 lanes x 4 pixels (16 bytes) of a row, of which
 // lanes 1..30 produce output and lanes 0 and 31 only supply the horizontal
-// halo (up to three pixels) by shuffle, and a band of at most kGauss8MaxBand
-// destination rows.  It requests every source row of the band at once (one
-// 16-byte cp.async per lane and row into its own shared-memory slots), in
-// copy groups of K rows that are filtered as they land, then streams down
-// the band: the unpacked rows of the vertical window stay in registers in
+// halo (up to three pixels) by shuffle, and a band of destination rows.  It
+// requests source rows in copy groups of K (one 16-byte cp.async per lane and
+// row into its own shared-memory slots, a ring of kRingRows) that are filtered
+// as they land.  Bands of 3x3 and 5x5 kernels are at most 14 rows, all of
+// whose source rows are requested at once; 7x7 bands, where 6 rows of halo on
+// 10 cost most, are up to 48 rows and keep three groups in flight down the
+// band (3840x2160 22.5 -> 21.6 us, 3841x2160 34.1 -> 29.8 us; the same for 5x5
+// and 3x3: 18.1 -> 18.8 us and 15.0 -> 15.8 us).  The unpacked rows of the vertical window stay in registers in
 // statically indexed slots (the row loop is unrolled by K).  The source rows
 // must be 4-byte aligned (whole pixels; other calls take the tiled kernel of
 // sepfused.cuh).  With 16-byte aligned rows, lanes whose 4 pixels lie inside the
@@ -46,9 +49,9 @@ constexpr int kThreadsG = 128;
 constexpr int kWarpsG = kThreadsG / 32;
 constexpr int kPix = 4;                            // pixels (16 bytes) per lane
 constexpr int kStripPix = kGauss8Lanes * kPix;     // destination pixels per strip
-constexpr int kStageRowsMax = kGauss8MaxBand + 6;  // source rows of a band, K <= 7
-constexpr int kWarpStage = kStageRowsMax * 32 * 16;
-constexpr int kSmemG = kWarpsG * kWarpStage;  // 40960
+constexpr int kRingRows = 21;                      // staged source rows: whole groups of 3, 5 (20) or 7
+constexpr int kWarpStage = kRingRows * 32 * 16;
+constexpr int kSmemG = kWarpsG * kWarpStage;  // 43008
 
 __device__ __forceinline__ void cp_async16g(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
@@ -58,7 +61,7 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait_g() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-// Waits until at most `pending` copy groups (0..7) are outstanding.
+// Waits until at most `pending` copy groups (0..5) are outstanding.
 __device__ __forceinline__ void cp_async_wait_upto(int pending) {
   switch (pending) {
     case 0: cp_async_wait_g<0>(); break;
@@ -66,17 +69,16 @@ __device__ __forceinline__ void cp_async_wait_upto(int pending) {
     case 2: cp_async_wait_g<2>(); break;
     case 3: cp_async_wait_g<3>(); break;
     case 4: cp_async_wait_g<4>(); break;
-    case 5: cp_async_wait_g<5>(); break;
-    case 6: cp_async_wait_g<6>(); break;
-    default: cp_async_wait_g<7>(); break;
+    default: cp_async_wait_g<5>(); break;
   }
 }
 
 template <int K>
 struct GaussGeo {
   static constexpr int R = K / 2;
-  static constexpr int kStageRows = kGauss8MaxBand + K - 1;
-  static constexpr int kGroups = (kStageRows + K - 1) / K;  // copy groups of K rows
+  static constexpr int kGroups = kRingRows / K;  // copy groups of K rows in the ring: 7, 4, 3
+  // Whether a band may outgrow the staged rows.
+  static constexpr bool kRing = gauss8_max_band(K) + K - 1 > kGroups * K;
 };
 
 // One lane's 4 pixels of a row as (channels 0, 2) and (channels 1, 3) words.
@@ -153,9 +155,9 @@ __device__ __forceinline__ void cp_async4g(uint32_t dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src));
 }
 
-template <int K, bool SIMPLE>
-__device__ __forceinline__ void band_loop8(const Gauss8Job &j, const uint4 *stage, int lane, int rows,
-                                           uint8_t *d, long e0, bool outputs, bool full_store);
+template <int K, bool SIMPLE, typename Copy>
+__device__ __forceinline__ void band_loop8(const Gauss8Job &j, const uint4 *stage, int lane, int rows, uint8_t *d,
+                                           long e0, bool outputs, bool full_store, Copy &&copy_group);
 
 template <int K>
 __device__ __forceinline__ void run_band8(const Gauss8Job &j, uint4 *stage, int strip, int band, int lane) {
@@ -180,30 +182,29 @@ __device__ __forceinline__ void run_band8(const Gauss8Job &j, uint4 *stage, int 
   const int y0 = band * j.band_q + min(band, j.band_r);
   const int y1 = y0 + rows;
   const int nrows = rows + K - 1;  // source rows y0 - R .. y1 + R - 1
-  // Request every source row: slot rr of the lane holds row y0 - R + rr, in
-  // groups of K rows ([gK, gK + K); empty groups at the end).
+  // Copy group g: source rows y0 - R + [gK, gK + K) into the lane's slots of
+  // ring group g % kGroups.
   const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(stage + lane));
-  if (fast && y0 >= R && y1 + R <= j.h) {
-    const uint8_t *g = j.src + static_cast<int64_t>(y0 - R) * j.src_stride + 4 * e0;
-    uint32_t a = sbase;
-    int rr = 0;
-#pragma unroll
-    for (int grp = 0; grp < G::kGroups; ++grp) {
+  const bool consecutive = fast && y0 >= R && y1 + R <= j.h;
+  auto copy_group = [&](int g) {
+    const int last = min(nrows, K * g + K);
+    const uint32_t first_slot = static_cast<uint32_t>(g % G::kGroups) * K;
+    if (K * g >= nrows) {
+      // Past the band: an empty group keeps the count.
+    } else if (consecutive) {
+      const uint8_t *p = j.src + static_cast<int64_t>(y0 - R + K * g) * j.src_stride + 4 * e0;
+      uint32_t a = sbase + first_slot * 512;
 #pragma unroll 1
-      for (; rr < min(nrows, K * grp + K); ++rr, a += 32 * 16, g += j.src_stride) cp_async16g(a, g);
-      cp_async_commit_g();
-    }
-  } else {
-    int rr = 0;
-#pragma unroll
-    for (int grp = 0; grp < G::kGroups; ++grp) {
+      for (int rr = K * g; rr < last; ++rr, a += 512, p += j.src_stride) cp_async16g(a, p);
+    } else {
+      uint32_t slot = first_slot;
 #pragma unroll 1
-      for (; rr < min(nrows, K * grp + K); ++rr) {
+      for (int rr = K * g; rr < last; ++rr, ++slot) {
         const int y = map_index(y0 - R + rr, j.h, j.border);
-        const uint32_t a = sbase + rr * 32 * 16;
+        const uint32_t a = sbase + slot * 512;
         if (y < 0 || !live) {
           // A CONSTANT border row, or a lane no stored pixel reads.
-          stage[rr * 32 + lane] = y < 0 ? make_uint4(bv4, bv4, bv4, bv4) : make_uint4(0u, 0u, 0u, 0u);
+          stage[slot * 32 + lane] = y < 0 ? make_uint4(bv4, bv4, bv4, bv4) : make_uint4(0u, 0u, 0u, 0u);
         } else {
           const uint8_t *row = j.src + static_cast<int64_t>(y) * j.src_stride;
           if (fast) {
@@ -214,25 +215,42 @@ __device__ __forceinline__ void run_band8(const Gauss8Job &j, uint4 *stage, int 
               if (col[k] >= 0)
                 cp_async4g(a + 4 * k, row + 4 * col[k]);
               else
-                reinterpret_cast<uint32_t *>(stage + rr * 32 + lane)[k] = bv4;
+                reinterpret_cast<uint32_t *>(stage + slot * 32 + lane)[k] = bv4;
             }
           }
         }
       }
+    }
+    cp_async_commit_g();
+  };
+  if (!G::kRing && consecutive) {
+    // The whole band at once: one walk down the rows.
+    const uint8_t *p = j.src + static_cast<int64_t>(y0 - R) * j.src_stride + 4 * e0;
+    uint32_t a = sbase;
+    int rr = 0;
+#pragma unroll
+    for (int grp = 0; grp < G::kGroups; ++grp) {
+#pragma unroll 1
+      for (; rr < min(nrows, K * grp + K); ++rr, a += 512, p += j.src_stride) cp_async16g(a, p);
       cp_async_commit_g();
     }
+  } else {
+#pragma unroll 1
+    for (int g = 0; g < G::kGroups; ++g) copy_group(g);
   }
   uint8_t *d = j.dst + static_cast<int64_t>(y0) * j.dst_stride + 4 * e0;
   // The byte-store path only where some lane of the warp needs it.
   if (__all_sync(0xffffffffu, !outputs || full_store))
-    band_loop8<K, true>(j, stage, lane, rows, d, e0, outputs, full_store);
+    band_loop8<K, true>(j, stage, lane, rows, d, e0, outputs, full_store, copy_group);
   else
-    band_loop8<K, false>(j, stage, lane, rows, d, e0, outputs, full_store);
+    band_loop8<K, false>(j, stage, lane, rows, d, e0, outputs, full_store, copy_group);
+  // The next item's copies follow into the same slots.
+  cp_async_wait_g<0>();
 }
 
-template <int K, bool SIMPLE>
-__device__ __forceinline__ void band_loop8(const Gauss8Job &j, const uint4 *stage, int lane, int rows,
-                                           uint8_t *d, long e0, bool outputs, bool full_store) {
+template <int K, bool SIMPLE, typename Copy>
+__device__ __forceinline__ void band_loop8(const Gauss8Job &j, const uint4 *stage, int lane, int rows, uint8_t *d,
+                                           long e0, bool outputs, bool full_store, Copy &&copy_group) {
   using G = GaussGeo<K>;
   constexpr int R = G::R;
   uint32_t wt[R + 1];
@@ -243,16 +261,22 @@ __device__ __forceinline__ void band_loop8(const Gauss8Job &j, const uint4 *stag
   cp_async_wait_g<G::kGroups - 1>();  // group 0: rows 0 .. K - 1
 #pragma unroll
   for (int rr = 0; rr < K - 1; ++rr) unpack4(stage[rr * 32 + lane], wl[rr], wh[rr]);
+  const uint4 *cur = stage + lane;  // the lane's slots of group `grp`
 #pragma unroll 1
-  for (int base = 0; base < rows; base += K) {
-    // Destination rows base .. base + K - 1 read source rows up to
-    // base + 2K - 2: groups up to base / K + 1.
-    cp_async_wait_upto(max(0, G::kGroups - 2 - base / K));
+  for (int base = 0, grp = 0; base < rows; base += K, ++grp) {
+    // Destination rows base .. base + K - 1 read source rows base + K - 1 ..
+    // base + 2K - 2: the last of group grp, whose slots then take group
+    // grp + kGroups, and all but the last of group grp + 1.
+    if (G::kRing) cp_async_wait_g<G::kGroups - 2>();
+    else cp_async_wait_upto(max(0, G::kGroups - 2 - grp));
+    const uint4 *const next = G::kRing ? stage + lane + (grp + 1) % G::kGroups * K * 32 : cur + K * 32;
     static_for<0, K>([&](auto sc) {
       constexpr int S = decltype(sc)::value;
       constexpr int slot = (S + K - 1) % K;  // receives source row base + S + K - 1
       if (base + S >= rows) return;  // past the band (the loop ends here)
-      unpack4(stage[(base + S + K - 1) * 32 + lane], wl[slot], wh[slot]);
+      unpack4(S == 0 ? cur[(K - 1) * 32] : next[(S - 1) * 32], wl[slot], wh[slot]);
+      if constexpr (S == 0)
+        if (G::kRing) copy_group(grp + G::kGroups);
       const uint4 out = filter_row8<K, S>(wl, wh, wt);
       if (SIMPLE) {
         if (outputs) *reinterpret_cast<uint4 *>(d) = out;
@@ -279,6 +303,7 @@ __device__ __forceinline__ void band_loop8(const Gauss8Job &j, const uint4 *stag
       }
       d += j.dst_stride;
     });
+    cur = next;
   }
 }
 
@@ -337,11 +362,11 @@ __global__ void __launch_bounds__(kThreadsG, K == 7 ? 4 : 5)
   }
 }
 
-// Bands of at most kGauss8MaxBand rows, as many as give `slots` warps the
+// Bands of at most gauss8_max_band rows, as many as give `slots` warps the
 // same number of items (one wave of n items per warp).
-void size_bands8(Gauss8Job &j, long slots) {
+void size_bands8(Gauss8Job &j, int ksize, long slots) {
   j.strips = (j.w + kStripPix - 1) / kStripPix;
-  const long min_bands = (j.h + kGauss8MaxBand - 1) / kGauss8MaxBand;
+  const long max_band = gauss8_max_band(ksize), min_bands = (j.h + max_band - 1) / max_band;
   const long per_warp = std::max(1L, (min_bands * j.strips + slots - 1) / slots);
   j.bands = static_cast<int32_t>(std::min<long>(j.h, std::max(min_bands, per_warp * slots / j.strips)));
   j.band_q = j.h / j.bands;
@@ -357,7 +382,7 @@ cudaError_t launch8(Gauss8Job &j, int sm_count, cudaStream_t stream) {
   const long resident = static_cast<long>(occ) * std::max(sm_count, 1);
   const long slots = resident * kWarpsG;
   // Every resident warp gets the same number of items.
-  size_bands8(j, slots);
+  size_bands8(j, K, slots);
   const long items = static_cast<long>(j.strips) * j.bands;
   const long grid = std::max(1L, std::min(resident, (items + kWarpsG - 1) / kWarpsG));
   cudaLaunchConfig_t cfg = {};
@@ -421,7 +446,7 @@ int gauss8_batch_warps(int ksize, int sm_count) {
   return 0;
 }
 
-void gauss8_size_for_share(Gauss8Job &j, int warps) { size_bands8(j, std::max(warps, 1)); }
+void gauss8_size_for_share(Gauss8Job &j, int ksize, int warps) { size_bands8(j, ksize, std::max(warps, 1)); }
 
 cudaError_t launch_gauss8_batch(int ksize, const Gauss8Job *table, int n, long items, int sm_count,
                                 cudaStream_t stream) {

@@ -115,9 +115,9 @@ struct Sep16Job {
 // Four-channel u8 Gaussians, 3x3 / 5x5 / 7x7 generated kernels summing to
 // 256 (csrc/gauss8.cu): a warp strip is 32 lanes x 4 pixels, of which
 // kGauss8Lanes lanes produce output; a warp item is (strip, band of at most
-// kGauss8MaxBand destination rows).
+// gauss8_max_band destination rows).
 constexpr int kGauss8Lanes = 30;
-constexpr int kGauss8MaxBand = 14;
+KCV_HD constexpr int gauss8_max_band(int ksize) { return ksize == 7 ? 48 : 14; }
 
 struct Gauss8Job {
   const uint8_t *src;

@@ -71,7 +71,7 @@ bool gauss8_eligible(const FilterJob &job);
 // a device table of n jobs of the same ksize holding `items` warp items.
 void gauss8_job(const FilterJob &f, Gauss8Job &j);
 int gauss8_batch_warps(int ksize, int sm_count);
-void gauss8_size_for_share(Gauss8Job &j, int warps);
+void gauss8_size_for_share(Gauss8Job &j, int ksize, int warps);
 cudaError_t launch_gauss8_batch(int ksize, const Gauss8Job *table, int n, long items, int sm_count,
                                 cudaStream_t stream);
 cudaError_t launch_gauss8(const FilterJob &job, int sm_count, cudaStream_t stream);
