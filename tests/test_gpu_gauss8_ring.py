@@ -1,6 +1,6 @@
 """The four-channel streaming Gaussian where its ring of staged rows can go
-wrong, against the CPU oracle: heights around multiples of the 7-row copy
-groups, of the 21-row ring and of a band's 48 rows, single calls and a plan
+wrong, against the CPU oracle: heights around multiples of the copy groups, of
+the rings (9, 20 and 14 rows) and of the bands (24, 14 and 48 rows), single calls and a plan
 (whose shares make the tallest bands), aligned, 4-byte aligned and border
 rows."""
 import numpy as np

@@ -15,12 +15,13 @@
 // lanes 1..30 produce output and lanes 0 and 31 only supply the horizontal
 // halo (up to three pixels) by shuffle, and a band of destination rows.  It
 // requests source rows in copy groups of K (one 16-byte cp.async per lane and
-// row into its own shared-memory slots, a ring of kRingRows) that are filtered
-// as they land.  Bands of 3x3 and 5x5 kernels are at most 14 rows, all of
-// whose source rows are requested at once; 7x7 bands, where 6 rows of halo on
-// 10 cost most, are up to 48 rows and keep three groups in flight down the
-// band (3840x2160 22.5 -> 21.6 us, 3841x2160 34.1 -> 29.8 us; the same for 5x5
-// and 3x3: 18.1 -> 18.8 us and 15.0 -> 15.8 us).  The unpacked rows of the vertical window stay in registers in
+// row into its own shared-memory slots) that are filtered as they land.  5x5
+// bands are at most 14 rows, all of whose source rows are requested at once.
+// 7x7 and 3x3 bands are taller (less halo to read again) and stage two or
+// three groups ahead in a ring: requesting less at once also lets every
+// warp's first rows arrive early.  3840x2160, source not in L2: 7x7 23.8 ->
+// 22.3 us, 3x3 17.0 -> 16.6 us; three groups of 7 23.8 us, 5x5 in a ring 20.1
+// instead of 19.8 us.  3841x2160 7x7 34.1 -> 29.9 us.  The unpacked rows of the vertical window stay in registers in
 // statically indexed slots (the row loop is unrolled by K).  The source rows
 // must be 4-byte aligned (whole pixels; other calls take the tiled kernel of
 // sepfused.cuh).  With 16-byte aligned rows, lanes whose 4 pixels lie inside the
@@ -49,9 +50,10 @@ constexpr int kThreadsG = 128;
 constexpr int kWarpsG = kThreadsG / 32;
 constexpr int kPix = 4;                            // pixels (16 bytes) per lane
 constexpr int kStripPix = kGauss8Lanes * kPix;     // destination pixels per strip
-constexpr int kRingRows = 21;                      // staged source rows: whole groups of 3, 5 (20) or 7
-constexpr int kWarpStage = kRingRows * 32 * 16;
-constexpr int kSmemG = kWarpsG * kWarpStage;  // 43008
+// Copy groups of K source rows staged at a time.
+constexpr int ring_groups(int k) { return k == 3 ? 3 : k == 5 ? 4 : 2; }
+constexpr int warp_stage8(int k) { return ring_groups(k) * k * 32 * 16; }  // bytes
+constexpr int smem8(int k) { return kWarpsG * warp_stage8(k); }
 
 __device__ __forceinline__ void cp_async16g(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
@@ -76,7 +78,7 @@ __device__ __forceinline__ void cp_async_wait_upto(int pending) {
 template <int K>
 struct GaussGeo {
   static constexpr int R = K / 2;
-  static constexpr int kGroups = kRingRows / K;  // copy groups of K rows in the ring: 7, 4, 3
+  static constexpr int kGroups = ring_groups(K);  // copy groups of K rows in the ring
   // Whether a band may outgrow the staged rows.
   static constexpr bool kRing = gauss8_max_band(K) + K - 1 > kGroups * K;
 };
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(kThreadsG, K == 7 ? 4 : 5) gauss8_kernel(const
   launch_dependents();
   grid_dependency_wait();  // the source may be the previous call's output
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint4 *stage = stage8 + warp * (kWarpStage / 16);
+  uint4 *stage = stage8 + warp * (warp_stage8(K) / 16);
   // Items go round the CTAs first, so that every SM gets the same number.
   const int gw = warp * gridDim.x + blockIdx.x;
   const int nw = gridDim.x * kWarpsG;
@@ -339,7 +341,7 @@ __global__ void __launch_bounds__(kThreadsG, K == 7 ? 4 : 5)
   extern __shared__ __align__(16) uint4 stage8b[];
   __shared__ int ends[kG8SearchEntries];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint4 *stage = stage8b + warp * (kWarpStage / 16);
+  uint4 *stage = stage8b + warp * (warp_stage8(K) / 16);
   const bool cached = n <= kG8SearchEntries;
   if (cached)
     for (int k = threadIdx.x; k < n; k += blockDim.x) ends[k] = E[k].item_end;
@@ -377,7 +379,7 @@ template <int K>
 cudaError_t launch8(Gauss8Job &j, int sm_count, cudaStream_t stream) {
   auto kern = gauss8_kernel<K>;
   int occ = 0;
-  const cudaError_t err = resident_ctas_per_sm<gauss8_kernel<K>>(kThreadsG, kSmemG, &occ);
+  const cudaError_t err = resident_ctas_per_sm<gauss8_kernel<K>>(kThreadsG, smem8(K), &occ);
   if (err != cudaSuccess) return err;
   const long resident = static_cast<long>(occ) * std::max(sm_count, 1);
   const long slots = resident * kWarpsG;
@@ -388,7 +390,7 @@ cudaError_t launch8(Gauss8Job &j, int sm_count, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(kThreadsG);
-  cfg.dynamicSmemBytes = kSmemG;
+  cfg.dynamicSmemBytes = smem8(K);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -411,7 +413,7 @@ bool gauss8_eligible(const FilterJob &f) {
 template <int K>
 int batch_warps8(int sm_count) {
   int occ = 0;
-  if (resident_ctas_per_sm<gauss8_batch_kernel<K>>(kThreadsG, kSmemG, &occ) != cudaSuccess) return 0;
+  if (resident_ctas_per_sm<gauss8_batch_kernel<K>>(kThreadsG, smem8(K), &occ) != cudaSuccess) return 0;
   return occ * std::max(sm_count, 1) * kWarpsG;
 }
 
@@ -420,7 +422,7 @@ cudaError_t launch_batch8(const Gauss8Job *table, int n, long items, int sm_coun
   const int warps = batch_warps8<K>(sm_count);
   if (warps == 0) return cudaErrorInvalidValue;
   const long grid = std::max(1L, std::min<long>(warps / kWarpsG, (items + kWarpsG - 1) / kWarpsG));
-  gauss8_batch_kernel<K><<<static_cast<unsigned>(grid), kThreadsG, kSmemG, stream>>>(table, n);
+  gauss8_batch_kernel<K><<<static_cast<unsigned>(grid), kThreadsG, smem8(K), stream>>>(table, n);
   return cudaGetLastError();
 }
 

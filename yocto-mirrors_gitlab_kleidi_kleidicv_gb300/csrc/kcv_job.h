@@ -117,7 +117,7 @@ struct Sep16Job {
 // kGauss8Lanes lanes produce output; a warp item is (strip, band of at most
 // gauss8_max_band destination rows).
 constexpr int kGauss8Lanes = 30;
-KCV_HD constexpr int gauss8_max_band(int ksize) { return ksize == 7 ? 48 : 14; }
+KCV_HD constexpr int gauss8_max_band(int ksize) { return ksize == 7 ? 48 : ksize == 5 ? 14 : 24; }
 
 struct Gauss8Job {
   const uint8_t *src;
