@@ -100,6 +100,19 @@ def test_separable_u8(c, taps):
                    rng, w, h, c, (0, 5, -w * c % 16)[n], 0, False)
 
 
+@pytest.mark.parametrize("k", [3, 5])
+@pytest.mark.parametrize("c", [1, 2, 3, 4])
+def test_binomial(k, c):
+    """Smaller images (any alignment) and larger ones on unaligned rows; the
+    last is large and aligned, which stays on the tiled stencil."""
+    rng = np.random.default_rng(10 * k + c)
+    for n, (w, h, pad) in enumerate([(k - 1, k - 1, 0), (256 // c, 32, 0), (256 // c + 1, 33, 1), (700, 65, 3),
+                                     (2049 // c, 2100, 1), (4096 // c, 1100, -(4096 // c) * c % 16)]):
+        for saturated in (False, True):
+            _gaussian(rng, w, h, c, k, 0.0, (FIXED + (kcv.CONSTANT,))[(n + c) % 5], pad=pad,
+                      ext=(n + c) % 5 == 4, saturated=saturated)
+
+
 def test_in_place_arbitrary_size_keeps_its_result():
     rng = np.random.default_rng(9)
     w, h, c, k = 300, 90, 3, 31

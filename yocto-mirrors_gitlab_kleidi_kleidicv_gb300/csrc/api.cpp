@@ -534,8 +534,8 @@ kleidicv_error_t execute(kleidicv_gpu_context *ctx, Prepared &p) {
       }
       Mma8Job mj;
       if (ctx->tune_threads <= 0 && mma8_job(p.fused, ctx->sm_count, mj)) {
-        // Other generated Gaussians and the u8 separable filter: the
-        // tensor-core stencil of mma8.cuh.
+        // Other generated Gaussians, the u8 separable filter and smaller or
+        // unaligned binomial 3x3 and 5x5: the tensor-core stencil of mma8.cuh.
         ctx->launches += 1;
         return cuda_status(ctx, launch_mma8(mj, ctx->sm_count, ctx->stream));
       }

@@ -11,8 +11,8 @@
 // on forked streams, so the groups run concurrently.  Blur-and-downsample
 // requests go to the pyramid kernel, four-channel generated 3x3 / 5x5 / 7x7
 // Gaussians to the streaming kernel of gauss8.cu and the other generated
-// Gaussians up to 15 taps and the u8 separable filter to the tensor-core
-// stencil of mma8.cuh (one launch per channel count, kernel size or
+// Gaussians up to 15 taps, the u8 separable filter and smaller or unaligned
+// binomial 3x3 and 5x5 to the tensor-core stencil of mma8.cuh (one launch per channel count, kernel size or
 // instantiation, over a job table): 512 images of 64..4096 x 64..2160 and 3 to
 // 15 taps 2373 -> 1056 us.  On the stencil the four-channel 3 / 5 / 7 taps of
 // that batch alone take 133 / 124 / 138 us against 75 / 75 / 109 us.

@@ -29,7 +29,8 @@ bool shape(Mma8Job &j) {
   j.tiles_x = (j.wc + j.tile_w - 1) / j.tile_w;
   j.tiles_y = (j.h + 16 * j.mt - 1) / (16 * j.mt);
   // 64: the last ldmatrix of a run may read one block past V.
-  const int rest = 256 * j.nk + 512 * j.nb + 16 * j.mt * j.v_pitch + 64;
+  const int planes = j.epi == kEpiBinomial ? 2 : 1;
+  const int rest = 256 * j.nk + planes * (512 * j.nb + 16 * j.mt * j.v_pitch) + 64;
   // All columns of a tile at once where two buffers of them fit, else in
   // equal chunks.
   const int cols = j.tile_w + 2 * (fixed ? mma8_round16(8 * (j.nb - 1)) : j.hp);
@@ -89,13 +90,21 @@ void common(const J &f, Mma8Job &j) {
 }  // namespace
 
 bool mma8_job(const FilterJob &f, int sm_count, Mma8Job &j) {
-  if (f.mode != MODE_SIGMA && f.mode != MODE_SEP_U8) return false;
+  // The binomial 3x3 and 5x5 need two planes of vertical results here, and the
+  // tiled stencil has cheap (constant) taps for them: it keeps the larger
+  // images whose rows TMA can load.  5x5, tiled against here: 320x240x1 8.5 /
+  // 4.1 us, 1920x1080x1 7.0 / 5.6 us, 1920x1080x3 9.6 / 9.9 us, 3840x2160x3 19.2
+  // / 23.3 us; unaligned rows 3841x2160x1 26.3 / 14.5 us, x4 60.3 / 43.9 us.
+  const bool unaligned = ((reinterpret_cast<uintptr_t>(f.src) | static_cast<uintptr_t>(f.src_stride)) & 15) != 0;
+  const bool binomial = f.mode == MODE_BINOM && f.ksize <= 5 &&
+                        (unaligned || static_cast<long>(f.width) * f.channels * f.height <= 4L << 20);
+  if (f.mode != MODE_SIGMA && f.mode != MODE_SEP_U8 && !binomial) return false;
   common(f, j);
   for (int t = 0; t < f.ksize; ++t) {
     j.ty[t] = static_cast<uint8_t>(f.wy[t]);
     j.tx[t] = static_cast<uint8_t>(f.wx[t]);
   }
-  j.epi = f.mode == MODE_SEP_U8 ? kEpiSat8 : kEpiRound;
+  j.epi = f.mode == MODE_SEP_U8 ? kEpiSat8 : binomial ? kEpiBinomial : kEpiRound;
   return plan(j, sm_count);
 }
 
@@ -124,6 +133,7 @@ namespace {
 // Instantiations with both step counts at compile time.
 cudaError_t launch_fixed(const Mma8Job &j, const Mma8Batch *batch, int sm_count, cudaStream_t stream) {
   if (j.epi == kEpiSat8) return launch_mma8_sat8(j, batch, sm_count, stream);
+  if (j.epi == kEpiBinomial) return launch_mma8_binomial(j, batch, sm_count, stream);
   switch (mma8_batch_key(j)) {
     case 121: return launch_mma8_1_2_1(j, batch, sm_count, stream);
     case 122: return launch_mma8_1_2_2(j, batch, sm_count, stream);
@@ -150,7 +160,7 @@ cudaError_t launch_mma8(const Mma8Job &j, int sm_count, cudaStream_t stream) {
 
 int mma8_batch_key(const Mma8Job &j) {
   if (!fixed_steps(j)) return 0;
-  return 1000 * (j.epi == kEpiSat8) + 100 * j.nk + 10 * j.nb + j.na;
+  return 1000 * j.epi + 100 * j.nk + 10 * j.nb + j.na;
 }
 
 bool mma8_batch_job(const FilterJob &f, Mma8Job &j) { return mma8_job(f, 0, j); }

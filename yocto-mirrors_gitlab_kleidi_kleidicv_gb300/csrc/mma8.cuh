@@ -1,5 +1,6 @@
 // u8 separable stencils on the tensor cores (sm_103a): gaussian_blur_u8 with
-// generated weights of any size (3..255) and the u8 separable filter.
+// generated weights of any size (3..255) and with the binomial kernels of
+// sizes 3 and 5, and the u8 separable filter.
 //
 // Both passes are products with a banded (Toeplitz) weight matrix, on
 // mma.sync.m16n8k16 (f16 operands, f32 accumulators):
@@ -81,8 +82,13 @@ __host__ __device__ constexpr int mma8_out_bytes(int run) { return kMma8Warps * 
 
 // How sums become bytes: bits 8..15 (weights sum to at most 256); the same
 // with the saturation and the right-border lanes of the arbitrary-size path;
-// min(sum, 255).
-enum Mma8Epi { kEpiRound = 0, kEpiArbitrary = 1, kEpiSat8 = 2 };
+// min(sum, 255); the binomial kernels of sizes 3 and 5, whose vertical sums
+// are not rounded (gaussian_blur_fixed_neon.cpp:27-153).  Those sums (at most
+// 1020 or 4080) are formed times 64 or 16, below 2^16, so that their high and
+// low bytes are byte results like the others; pass 2 multiplies the planes of
+// high and low bytes with the weights times 64 (16) and divided by 4 (16), all
+// exact, which gives 16 (1) times the binomial sum.
+enum Mma8Epi { kEpiRound = 0, kEpiArbitrary = 1, kEpiSat8 = 2, kEpiBinomial = 3 };
 
 __host__ __device__ constexpr int mma8_round16(int v) { return (v + 15) / 16 * 16; }
 // Row pitch: an odd multiple of 16 bytes.
@@ -152,11 +158,10 @@ __device__ __forceinline__ uint32_t odd_bytes(uint32_t w) { return __byte_perm(w
 // The accumulators' first value.  Four opaque registers: as known constants
 // they are copied into place before every first mma (four moves each, a
 // sixth of the kernel's instructions).
-template <int EPI>
+template <bool ROUND>
 __device__ __forceinline__ void mma8_init(float (&c)[4]) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    asm volatile("mov.b32 %0, %1;" : "=f"(c[i]) : "n"(EPI == kEpiSat8 ? 0x3F000000 : 0x3F000080));
+  for (int i = 0; i < 4; ++i) asm volatile("mov.b32 %0, %1;" : "=f"(c[i]) : "n"(ROUND ? 0x3F000080 : 0x3F000000));
 }
 // The result bytes of two sums in the low half of a word.
 template <int EPI>
@@ -186,7 +191,7 @@ struct Mma8Taps {
   uint8_t y[kTapsY], x[kTapsX];
 };
 
-// Integers 0..255 as f16: 1024 + v placed by its bits, minus 1024 (exact).
+// Integers 0..1023 as f16: 1024 + v placed by its bits, minus 1024 (exact).
 __device__ __forceinline__ uint32_t half_pair(uint32_t lo, uint32_t hi) {
   const uint32_t biased = 0x64006400u | lo | hi << 16, bias = 0x64006400u;
   const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&biased), *reinterpret_cast<const __half2 *>(&bias));
@@ -202,20 +207,31 @@ __device__ __forceinline__ void spread_taps(const Mma8Job &j, Mma8Taps &taps) {
     taps.x[kTapPad + i * j.c] = j.tx[i];
   }
 }
+template <int EPI>
 __device__ __forceinline__ void build_weights(const Mma8Job &j, const Mma8Taps &taps, uint32_t *wa, uint32_t *wb) {
   const int na = j.nk * 64, n = na + j.nb * 128;
+  // Binomial: the vertical weights and those of the high plane times `up`, the
+  // low plane's (behind them) times `down`.
+  const uint32_t up = EPI == kEpiBinomial ? (j.ksize == 3 ? 64u : 16u) : 1u;
+  const __half2 down = __float2half2_rn(j.ksize == 3 ? 0.25f : 0.0625f);
   for (int i = threadIdx.x; i < n; i += kMma8Threads) {
     if (i < na) {
       // B[k][n]: destination row n = g, source rows k = 2t, 2t + 1 (+ 8 in word 1).
       const int l = (i >> 1) & 31, g = l >> 2, t = l & 3;
       const int z = min(16 * (i >> 6) + 2 * t + (i & 1) * 8 - g, 2 * j.r + 1);
-      wa[i] = half_pair(taps.y[kTapPad + z], taps.y[kTapPad + z + 1]);
+      wa[i] = half_pair(up * taps.y[kTapPad + z], up * taps.y[kTapPad + z + 1]);
     } else {
       // B[k][n] of accumulator p: destination byte n + 8p, k = bytes 4t + e and
       // 4t + e + 2 of the step's block (e = word & 1).
       const int w = i - na, l = (w >> 2) & 31, g = l >> 2, t = l & 3;
       const int z = min(16 * (w >> 7) + 4 * t + (w & 1) - j.vo - (g + 4 * (w & 2)) + j.rc, 2 * j.rc + 1);
-      wb[w] = half_pair(taps.x[kTapPad + z], taps.x[kTapPad + z + 2]);
+      const uint32_t lo = taps.x[kTapPad + z], hi = taps.x[kTapPad + z + 2];
+      wb[w] = half_pair(up * lo, up * hi);
+      if constexpr (EPI == kEpiBinomial) {
+        const uint32_t h = half_pair(lo, hi);
+        const __half2 q = __hmul2(*reinterpret_cast<const __half2 *>(&h), down);
+        wb[j.nb * 128 + w] = *reinterpret_cast<const uint32_t *>(&q);
+      }
     }
   }
 }
@@ -364,7 +380,7 @@ __device__ __forceinline__ void vertical_pass(const Mma8Job &j, const Mma8Smem &
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   float init[4];
-  mma8_init<EPI>(init);
+  mma8_init<EPI == kEpiRound || EPI == kEpiArbitrary>(init);
   const uint2 *wa = reinterpret_cast<const uint2 *>(s.wa);
   const int rp = G::raw_pitch(j), vp = G::v_pitch(j);
   const uint32_t raw = smem_addr(s.raw) + lane * rp;  // the lane's row of ldmatrix loads
@@ -373,6 +389,15 @@ __device__ __forceinline__ void vertical_pass(const Mma8Job &j, const Mma8Smem &
   const bool sat = EPI == kEpiArbitrary && j.saturate != 0;
   auto store = [&](const float (&acc)[4], int group, uint32_t v) {
     v += 8 * group * vp;
+    if constexpr (EPI == kEpiBinomial) {
+      const uint32_t c[4] = {__float_as_uint(acc[0]), __float_as_uint(acc[1]), __float_as_uint(acc[2]),
+                             __float_as_uint(acc[3])};
+      sts16(v, __byte_perm(c[0], c[2], 0x0051));
+      sts16(v + vp, __byte_perm(c[1], c[3], 0x0051));
+      sts16(v + 16 * MT * vp, __byte_perm(c[0], c[2], 0x0040));
+      sts16(v + 16 * MT * vp + vp, __byte_perm(c[1], c[3], 0x0040));
+      return;
+    }
     sts16(v, pack_pair<EPI>(finish_sum<EPI>(acc[0], sat), finish_sum<EPI>(acc[2], sat)));
     sts16(v + vp, pack_pair<EPI>(finish_sum<EPI>(acc[1], sat), finish_sum<EPI>(acc[3], sat)));
   };
@@ -553,7 +578,7 @@ __device__ __forceinline__ void horizontal_pass(const Mma8Job &j, const Mma8Smem
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   float init[4];
-  mma8_init<EPI>(init);
+  mma8_init<EPI != kEpiSat8>(init);
   const uint4 *wb = reinterpret_cast<const uint4 *>(s.wb);
   const int vp = Mma8Geo<NK, NB, MT, W>::v_pitch(j);
   constexpr int RUN = mma8_run(MT, W), kBlocks = RUN / 16, kPitch = mma8_out_pitch(RUN);
@@ -604,17 +629,28 @@ __device__ __forceinline__ void horizontal_pass(const Mma8Job &j, const Mma8Smem
         const uint4 w = wb[k * 32 + lane];
         wr[k][0] = w.x, wr[k][1] = w.y, wr[k][2] = w.z, wr[k][3] = w.w;
       }
-      // win[k % (NB + 1)]: the A operand of block k, loaded in pairs.
-      uint32_t win[NB + 1][4];
+      // win[k % (NB + 1)]: the A operand of block k, loaded in pairs; of the
+      // plane of low bytes in wlo with its weights wrl.
+      constexpr bool kPlanes = EPI == kEpiBinomial;
+      uint32_t win[NB + 1][4], wlo[kPlanes ? NB + 1 : 1][4], wrl[kPlanes ? NB : 1][4];
+      if constexpr (kPlanes) {
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+          const uint4 w = wb[(NB + k) * 32 + lane];
+          wrl[k][0] = w.x, wrl[k][1] = w.y, wrl[k][2] = w.z, wrl[k][3] = w.w;
+        }
+      }
       float accs[2][2][4];
       auto load_pair = [&](auto kc) {
         constexpr int k = decltype(kc)::value;
-        uint32_t r[4];
-        ldsm_x4(r, va + 16 * k);
-        uint32_t(&w0)[4] = win[k % (NB + 1)];
-        uint32_t(&w1)[4] = win[(k + 1) % (NB + 1)];
-        w0[0] = even_bytes(r[0]), w0[1] = even_bytes(r[1]), w0[2] = odd_bytes(r[0]), w0[3] = odd_bytes(r[1]);
-        w1[0] = even_bytes(r[2]), w1[1] = even_bytes(r[3]), w1[2] = odd_bytes(r[2]), w1[3] = odd_bytes(r[3]);
+        auto load = [&](uint32_t addr, uint32_t(&w0)[4], uint32_t(&w1)[4]) {
+          uint32_t r[4];
+          ldsm_x4(r, addr);
+          w0[0] = even_bytes(r[0]), w0[1] = even_bytes(r[1]), w0[2] = odd_bytes(r[0]), w0[3] = odd_bytes(r[1]);
+          w1[0] = even_bytes(r[2]), w1[1] = even_bytes(r[3]), w1[2] = odd_bytes(r[2]), w1[3] = odd_bytes(r[3]);
+        };
+        load(va + 16 * k, win[k % (NB + 1)], win[(k + 1) % (NB + 1)]);
+        if constexpr (kPlanes) load(va + 16 * MT * vp + 16 * k, wlo[k % (NB + 1)], wlo[(k + 1) % (NB + 1)]);
       };
       // Blocks 0 .. NB - 2 before the first output block.
       static_for<0, NB - 1>([&](auto kc) {
@@ -633,6 +669,11 @@ __device__ __forceinline__ void horizontal_pass(const Mma8Job &j, const Mma8Smem
           } else {
             if constexpr (k < NA) mma_f16(acc[0], a, wr[k][0], wr[k][1]);
             mma_f16(acc[1], a, wr[k][2], wr[k][3]);
+          }
+          if constexpr (kPlanes) {
+            const uint32_t(&al)[4] = wlo[(b + k) % (NB + 1)];
+            if constexpr (k < NA) mma_f16(acc[0], al, wrl[k][0], wrl[k][1]);
+            mma_f16(acc[1], al, wrl[k][2], wrl[k][3]);
           }
         });
         // A block's results are staged behind the next block's products.
@@ -709,7 +750,7 @@ __device__ __forceinline__ void mma8_tiles(const Mma8Job &j, Mma8Taps &taps, uin
   Mma8Smem s;
   s.wa = reinterpret_cast<uint32_t *>(mem8);
   s.wb = s.wa + (G::kFixed ? NK : j.nk) * 64;
-  uint8_t *const raw0 = reinterpret_cast<uint8_t *>(s.wb + (G::kFixed ? NB : j.nb) * 128);
+  uint8_t *const raw0 = reinterpret_cast<uint8_t *>(s.wb + (G::kFixed ? NB : j.nb) * 128 * (EPI == kEpiBinomial ? 2 : 1));
   const int raw_bytes = max(G::raw_rows(j) * G::raw_pitch(j), mma8_out_bytes(mma8_run(MT, W)));
   s.raw = raw0;
   s.v = raw0 + 2 * raw_bytes;
@@ -728,7 +769,7 @@ __device__ __forceinline__ void mma8_tiles(const Mma8Job &j, Mma8Taps &taps, uin
   spread_taps(j, taps);
   stage(s.raw);
   __syncthreads();
-  build_weights(j, taps, s.wa, s.wb);
+  build_weights<EPI>(j, taps, s.wa, s.wb);
   while (count > 0) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();

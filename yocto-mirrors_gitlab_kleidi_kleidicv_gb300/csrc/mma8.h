@@ -32,7 +32,8 @@ bool mma8_batch_job(const FilterJob &f, Mma8Job &j);
 cudaError_t launch_mma8_batch(const Mma8Job &rep, const Mma8Batch &b, int sm_count, cudaStream_t stream);
 
 // Instantiations, one translation unit each: <vertical steps>_<horizontal
-// steps nb>_<na>, or any number of steps; the u8 separable filter.
+// steps nb>_<na>, or any number of steps; the u8
+// separable filter; the binomial kernels of sizes 3 and 5.
 cudaError_t launch_mma8_1_2_1(const Mma8Job &j, const Mma8Batch *batch, int sm_count, cudaStream_t stream);
 cudaError_t launch_mma8_1_2_2(const Mma8Job &j, const Mma8Batch *batch, int sm_count, cudaStream_t stream);
 cudaError_t launch_mma8_1_3_2(const Mma8Job &j, const Mma8Batch *batch, int sm_count, cudaStream_t stream);
@@ -47,6 +48,7 @@ cudaError_t launch_mma8_3_4_3(const Mma8Job &j, const Mma8Batch *batch, int sm_c
 cudaError_t launch_mma8_2_any(const Mma8Job &j, int sm_count, cudaStream_t stream);
 cudaError_t launch_mma8_3_any(const Mma8Job &j, int sm_count, cudaStream_t stream);
 cudaError_t launch_mma8_0_any(const Mma8Job &j, int sm_count, cudaStream_t stream);
+cudaError_t launch_mma8_binomial(const Mma8Job &j, const Mma8Batch *batch, int sm_count, cudaStream_t stream);
 cudaError_t launch_mma8_sat8(const Mma8Job &j, const Mma8Batch *batch, int sm_count, cudaStream_t stream);
 
 }  // namespace kcv
