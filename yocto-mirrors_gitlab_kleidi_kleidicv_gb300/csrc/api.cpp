@@ -539,6 +539,10 @@ kleidicv_error_t execute(kleidicv_gpu_context *ctx, Prepared &p) {
         ctx->launches += 1;
         return cuda_status(ctx, launch_mma8(mj, ctx->sm_count, ctx->stream));
       }
+      if (ctx->tune_threads <= 0 && sobel_eligible(p.fused)) {
+        ctx->launches += 1;
+        return cuda_status(ctx, launch_sobel(p.fused, ctx->stream));
+      }
       if (ctx->tune_threads <= 0 && sep16_eligible(p.fused)) {
         // One-channel 16-bit 5x5: the fp32 streaming kernel of sep16.cu.
         ctx->launches += 1;

@@ -76,6 +76,11 @@ cudaError_t launch_gauss8_batch(int ksize, const Gauss8Job *table, int n, long i
                                 cudaStream_t stream);
 cudaError_t launch_gauss8(const FilterJob &job, int sm_count, cudaStream_t stream);
 
+// Sobel 3x3 derivatives of smaller images and of unaligned rows
+// (csrc/sobel.cu).
+bool sobel_eligible(const FilterJob &job);
+cudaError_t launch_sobel(const FilterJob &job, cudaStream_t stream);
+
 // blur_and_downsample_u8 levels (csrc/pyramid.cu): one launch per phase, in
 // order.
 cudaError_t launch_pyramid(const PyrLaunch &L, int sm_count, cudaStream_t stream);
