@@ -166,14 +166,16 @@ __device__ __forceinline__ uint32_t med3(uint32_t a, uint32_t b, uint32_t c) {
 // output rows: the median of nine is the median of the largest minimum, the
 // median middle and the smallest maximum of the window's rows.  Packed: rows r
 // and r + 2 share a word, 12 minima and maxima per element (18 otherwise) where
-// selecting from each window took 42.  Measured: u8 1920x1080x1 14.4 -> 9.4 us,
-// 160x120x3 4.2 -> 4.1 us; f32 1280x720x3 18.6 -> 12.4 us (the kernel below, at
+// selecting from each window took 42.  Measured: u8 1920x1080x1 14.4 -> 7.1 us,
+// 160x120x1 4.2 -> 3.8 us; f32 1280x720x3 18.6 -> 12.4 us (the kernel below, at
 // K = 3: 8.3, 6.3 and 20.5 us).  Bound by its 4.5 loads per element.
 template <typename T>
 __global__ void __launch_bounds__(128) median3_kernel(const uint8_t *src, int64_t src_stride, uint8_t *dst,
                                                       int64_t dst_stride, int w, int h, int c, int border) {
   constexpr bool PACKED = sizeof(T) <= 2;
   constexpr int N = PACKED ? 4 : 6;  // sorted rows
+  launch_dependents();
+  grid_dependency_wait();  // the source may be the previous call's output
   const int xe = blockIdx.x * blockDim.x + threadIdx.x;  // element index in the row
   if (xe >= w * c) return;
   const int col = xe / c, ch = xe - col * c;
@@ -230,8 +232,8 @@ __global__ void __launch_bounds__(128) median3_kernel(const uint8_t *src, int64_
 // selection network takes the median of what is left: about 50 half-rate minima
 // and maxima per element (packed: two elements) at K = 5, where selecting from
 // each window by itself took 330.  Measured (1920x1080x1): u8 K = 5 / 7 49.4 /
-// 152 -> 14.5 / 28.8 us, f32 K = 5 49.4 -> 21.6 us; 160x120 K = 5 6.2 -> 4.3 us.
-// Bound by the networks' instructions (6 us of 14.5 at K = 5) and the staging's
+// 152 -> 12.1 / 26.5 us, f32 K = 5 49.4 -> 20.0 us; 160x120 K = 5 6.2 -> 3.8 us.
+// Bound by the networks' instructions (6 us of 12.1 at K = 5) and the staging's
 // loads and 16-bit stores.
 constexpr int median_width(int k) { return k == 7 ? 2 : 4; }  // pixels of a lane
 constexpr int median_pitch(int k) { return (32 * median_width(k) + k - 1 + 3) / 4 * 4; }
@@ -304,6 +306,8 @@ __global__ void __launch_bounds__(128)
   // All channels in a block, or one per grid layer.
   const int channels = gridDim.z > 1 ? 1 : c, c0 = blockIdx.z;
   extern __shared__ __align__(16) uint32_t median_mem[];
+  launch_dependents();
+  grid_dependency_wait();  // the source may be the previous call's output
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int x0 = blockIdx.x * TX;
   // Row blocks loop over the grid's y extent, which the hardware caps at 65535.
@@ -422,6 +426,8 @@ __global__ void __launch_bounds__(kHistThreads) median_hist_kernel(const uint8_t
                                                                   int h, int c, int k,
                                                                   int border, int run) {
   __shared__ uint16_t hist[256 * kHistThreads];  // [bin][thread]; counts <= 255 * 255
+  launch_dependents();
+  grid_dependency_wait();  // the source may be the previous call's output
   const int tid = threadIdx.x;
   const int g = blockIdx.x * kHistThreads + tid;  // (segment, channel) item of a row
   const int ch = g % c, seg = g / c;
@@ -457,6 +463,22 @@ __global__ void __launch_bounds__(kHistThreads) median_hist_kernel(const uint8_t
   }
 }
 
+// Launch under programmatic dependent launch, as the other single calls.
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 template <typename T, int K>
 cudaError_t launch_small(const MedianJob &j, cudaStream_t s) {
   constexpr bool PACKED = sizeof(T) <= 2;
@@ -474,9 +496,8 @@ cudaError_t launch_small(const MedianJob &j, cudaStream_t s) {
   // At most 38,016 bytes (packed, four channels, K = 5).
   const size_t smem =
       sizeof(uint32_t) * (j.channels / layers) * median_stage_rows(rows, K, PACKED) * median_pitch(K);
-  median_small_kernel<T, K><<<grid, 128, smem, s>>>(j.src, j.src_stride, j.dst, j.dst_stride, j.width, j.height,
-                                                           j.channels, j.border, rows);
-  return cudaGetLastError();
+  return launch_early(median_small_kernel<T, K>, grid, 128, smem, s, j.src, j.src_stride, j.dst, j.dst_stride,
+                      j.width, j.height, j.channels, j.border, rows);
 }
 
 template <typename T>
@@ -484,9 +505,8 @@ cudaError_t launch3(const MedianJob &j, cudaStream_t s) {
   const int row_blocks = (j.height + 3) / 4;
   dim3 grid(static_cast<unsigned>((j.width * j.channels + 127) / 128),
             static_cast<unsigned>(row_blocks < 65535 ? row_blocks : 65535));
-  median3_kernel<T><<<grid, 128, 0, s>>>(j.src, j.src_stride, j.dst, j.dst_stride, j.width, j.height, j.channels,
-                                         j.border);
-  return cudaGetLastError();
+  return launch_early(median3_kernel<T>, grid, 128, 0, s, j.src, j.src_stride, j.dst, j.dst_stride, j.width, j.height,
+                      j.channels, j.border);
 }
 
 template <typename T>
@@ -508,10 +528,8 @@ cudaError_t launch_median(const MedianJob &j, cudaStream_t s) {
     const int items = j.channels * ((j.width + run - 1) / run);
     dim3 grid(static_cast<unsigned>((items + kHistThreads - 1) / kHistThreads),
               static_cast<unsigned>(j.height < 65535 ? j.height : 65535));
-    median_hist_kernel<<<grid, kHistThreads, 0, s>>>(j.src, j.src_stride, j.dst, j.dst_stride,
-                                                     j.width, j.height, j.channels, j.ksize,
-                                                     j.border, run);
-    return cudaGetLastError();
+    return launch_early(median_hist_kernel, grid, kHistThreads, 0, s, j.src, j.src_stride, j.dst, j.dst_stride,
+                        j.width, j.height, j.channels, j.ksize, j.border, run);
   }
   switch (j.elem) {
     case MEDIAN_S8: return launch_typed<int8_t>(j, s);
