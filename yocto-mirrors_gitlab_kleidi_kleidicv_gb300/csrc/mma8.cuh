@@ -805,7 +805,7 @@ __device__ __forceinline__ void mma8_tiles(const Mma8Job &j, Mma8Taps &taps, uin
 }
 
 template <int NK, int NB, int NA, int MT, int W, int EPI>
-__global__ void __launch_bounds__(kMma8Threads, NK != 1 ? 2 : 3) mma8_kernel(const __grid_constant__ Mma8Job j) {
+__global__ void __launch_bounds__(kMma8Threads, 2) mma8_kernel(const __grid_constant__ Mma8Job j) {
   extern __shared__ __align__(16) uint8_t mem8[];
   __shared__ __align__(4) Mma8Taps taps;
   launch_dependents();
@@ -819,7 +819,7 @@ __global__ void __launch_bounds__(kMma8Threads, NK != 1 ? 2 : 3) mma8_kernel(con
 // which job k holds the tiles [ends[k - 1], ends[k]).  CTAs claim runs of
 // `chunk` tiles through *next (0 at launch).
 template <int NK, int NB, int NA, int MT, int W, int EPI>
-__global__ void __launch_bounds__(kMma8Threads, NK != 1 ? 2 : 3)
+__global__ void __launch_bounds__(kMma8Threads, 2)
     mma8_batch_kernel(const Mma8Job *__restrict__ jobs, const int *__restrict__ ends, int n, int chunk, int *next) {
   extern __shared__ __align__(16) uint8_t mem8[];
   __shared__ __align__(4) Mma8Taps taps;
