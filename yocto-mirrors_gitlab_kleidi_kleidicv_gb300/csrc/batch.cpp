@@ -14,7 +14,7 @@
 // Gaussians up to 15 taps, the u8 separable filter and smaller or unaligned
 // binomial 3x3 and 5x5 to the tensor-core stencil of mma8.cuh (one launch per channel count, kernel size or
 // instantiation, over a job table): 512 images of 64..4096 x 64..2160 and 3 to
-// 15 taps 2373 -> 1056 us.  On the stencil the four-channel 3 / 5 / 7 taps of
+// 15 taps 2373 -> 942 us.  On the stencil the four-channel 3 / 5 / 7 taps of
 // that batch alone take 133 / 124 / 138 us against 75 / 75 / 109 us.
 // Arbitrary-size Gaussians and copies run on a branch of their own.  With
 // use_graph the whole launch is captured once into a CUDA graph and replayed.

@@ -54,7 +54,8 @@ bool plan(Mma8Job &j, int sm_count) {
   j.na = (j.vo + 8 + j.rc + 15) / 16;
   // 64 x 256 bytes where that gives every SM two tiles, else 32 x 256:
   // 3840x2160x1 7 taps 7.7 us against 8.4 us, 1920x1080x1 5.8 us against
-  // 4.7 us, 640x480x1 4.1 us against 3.6 us (16 x 128 gained nothing there).
+  // 4.7 us, 640x480x1 4.1 us against 3.6 us (16 x 128 gained nothing there;
+  // all with three CTAs per SM).
   j.tile_w = 256;
   for (j.mt = 4;; j.mt = 2) {
     if (!shape(j)) return false;
@@ -93,7 +94,7 @@ bool mma8_job(const FilterJob &f, int sm_count, Mma8Job &j) {
   // The binomial 3x3 and 5x5 need two planes of vertical results here, and the
   // tiled stencil has cheap (constant) taps for them: it keeps the larger
   // images whose rows TMA can load.  5x5, tiled against here: 320x240x1 8.5 /
-  // 4.1 us, 1920x1080x1 7.0 / 5.6 us, 1920x1080x3 9.6 / 9.9 us, 3840x2160x3 19.2
+  // 3.9 us, 1920x1080x1 7.0 / 4.5 us, 1920x1080x3 9.6 / 9.9 us, 3840x2160x3 19.2
   // / 23.3 us; unaligned rows 3841x2160x1 26.3 / 14.5 us, x4 60.3 / 43.9 us.
   const bool unaligned = ((reinterpret_cast<uintptr_t>(f.src) | static_cast<uintptr_t>(f.src_stride)) & 15) != 0;
   const bool binomial = f.mode == MODE_BINOM && f.ksize <= 5 &&

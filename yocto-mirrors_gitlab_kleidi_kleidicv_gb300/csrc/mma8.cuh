@@ -56,11 +56,15 @@
 // pass 2.
 //
 // Measured (GB300, back to back; before: the tiled and the two-pass kernel):
-// 3840x2160x1 31 taps 132 -> 10.5 us, 255 taps 873 -> 77 us; 3840x2160x3 15
-// taps 66 -> 22.9 us, 1917x1079x3 (unaligned rows) 48.3 -> 14.3 us;
-// 3840x2160x4 21 taps 134 -> 42.9 us; 1920x1080x1 7 taps 9.3 -> 4.7 us.  At 7
-// taps bound by issue (about 190 warp instructions per 16 x 16 bytes and 0.5
-// per scheduler and cycle), from about 100 taps on by the tensor pipe.
+// 3840x2160x1 31 taps 132 -> 10.7 us, 255 taps 873 -> 77 us; 3840x2160x3 15
+// taps 66 -> 22.9 us, 1917x1079x3 (unaligned rows) 48.3 -> 13.9 us;
+// 3840x2160x4 21 taps 134 -> 43.1 us; 1920x1080x1 7 taps 9.3 -> 4.1 us.
+// Bound by latency at too few warps, not by a pipe: 3840x2160x1 at 7 / 31 /
+// 101 / 255 taps uses 44 / 42 / 34 / 33 % of the issue slots and 19 / 34 / 37 /
+// 43 % of the tensor pipe's cycles, with 25 % of the warps resident, and 14 %
+// (shared memory for one CTA) at 101 and 255 taps.  Three CTAs of 72
+// registers per thread spill: 1920x1080x1 7 taps 4.9 us.  7 taps are 99 warp
+// instructions per 16 x 16 bytes; unaligned rows take 1.7 times as many.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -283,9 +287,11 @@ __device__ __forceinline__ void stage_pieces(const Mma8Job &j, uint8_t *raw, int
   } else {
     // The two aligned blocks around the piece, where they lie in the image
     // (bytes of the neighbouring rows are replaced or never read), loaded for
-    // three rows before the first is shifted and stored.
+    // two rows before the first is shifted and stored.  The 512-image batch with
+    // 1 / 2 / 3 / 5 rows: 998 / 942 / 988 / 1204 us; the batch kernels spill up
+    // to 32 / 84 / 224 bytes at 2 / 3 / 5.
     const uint8_t *const end = j.src + static_cast<int64_t>(j.h - 1) * j.src_stride + j.wc;
-    constexpr int kAhead = 3;
+    constexpr int kAhead = 2;
     for (int row = row0; row < rows; row += kAhead * step, off += kAhead * step * pitch) {
       uint4 u[kAhead], v[kAhead];
       int sh[kAhead];  // -1: nothing loaded
