@@ -131,3 +131,18 @@ def test_block_edges(dtype, k):
                                 seed=100 * k + n, pad=n % 3, dpad=n % 2, ctx=ctx)
         assert pad_ok and np.array_equal(got, want), (w, h, c)
     ctx.close()
+
+
+@pytest.mark.parametrize("dtype", ["u8", "s16", "f32"])
+@pytest.mark.parametrize("k", [5, 7])
+def test_channel_layers(dtype, k):
+    """Several channels on both sides of the line below which every channel has
+    blocks of its own, at each number of rows of a block (u8: 4, 8, 16, 16; then
+    all channels in a block)."""
+    ctx = kcv.Context.for_torch(0)
+    size = np.dtype(oracle.MEDIAN_DTYPES[dtype]).itemsize  # a source is aligned to its element
+    for n, (w, h, c) in enumerate([(257, 131, 2), (513, 161, 3), (641, 257, 4), (1023, 767, 3), (1025, 769, 2)]):
+        got, want, pad_ok = run(dtype, w, h, c, k, (kcv.REVERSE, kcv.WRAP, kcv.REFLECT, kcv.REPLICATE)[n % 4],
+                                seed=500 * k + n, pad=n % 3, soff=n % 2 * size, dpad=n % 2, ctx=ctx)
+        assert pad_ok and np.array_equal(got, want), (w, h, c)
+    ctx.close()

@@ -168,7 +168,8 @@ __device__ __forceinline__ uint32_t med3(uint32_t a, uint32_t b, uint32_t c) {
 // and r + 2 share a word, 12 minima and maxima per element (18 otherwise) where
 // selecting from each window took 42.  Measured: u8 1920x1080x1 14.4 -> 7.1 us,
 // 160x120x1 4.2 -> 3.8 us; f32 1280x720x3 18.6 -> 12.4 us (the kernel below, at
-// K = 3: 8.3, 6.3 and 20.5 us).  Bound by its 4.5 loads per element.
+// K = 3: 8.3, 6.3 and 20.5 us).  Bound by issue: 68 % of the slots and half of
+// the ALU pipe, 18 % of the load pipe, 74 % of the warps resident.
 template <typename T>
 __global__ void __launch_bounds__(128) median3_kernel(const uint8_t *src, int64_t src_stride, uint8_t *dst,
                                                       int64_t dst_stride, int w, int h, int c, int border) {
@@ -233,8 +234,10 @@ __global__ void __launch_bounds__(128) median3_kernel(const uint8_t *src, int64_
 // and maxima per element (packed: two elements) at K = 5, where selecting from
 // each window by itself took 330.  Measured (1920x1080x1): u8 K = 5 / 7 49.4 /
 // 152 -> 12.1 / 26.5 us, f32 K = 5 49.4 -> 20.0 us; 160x120 K = 5 6.2 -> 3.8 us.
-// Bound by the networks' instructions (6 us of 12.1 at K = 5) and the staging's
-// loads and 16-bit stores.
+// Bound by latency with few warps: half of the ALU pipe and 40 % of the issue
+// slots at 16 % of the warps resident (three blocks of up to 168 registers).  Four
+// blocks of 128 registers spill: u8 1920x1080x3 K = 5 32.1 -> 28.3 us, but
+// 1280x720x1 5.6 -> 7.8 us and u16 1920x1080x1 11.9 -> 13.5 us.
 constexpr int median_width(int k) { return k == 7 ? 2 : 4; }  // pixels of a lane
 constexpr int median_pitch(int k) { return (32 * median_width(k) + k - 1 + 3) / 4 * 4; }
 constexpr int median_group(bool packed) { return packed ? 4 : 2; }  // output rows of a lane
@@ -484,13 +487,22 @@ cudaError_t launch_small(const MedianJob &j, cudaStream_t s) {
   constexpr bool PACKED = sizeof(T) <= 2;
   constexpr int tx = 32 * median_width(K), group = median_group(PACKED);
   const int columns = (j.width + tx - 1) / tx;
-  // Four warps on 4 groups of rows; fewer groups (all warps still stage) for
-  // images that would give the GPU less than two such blocks per SM.
+  auto blocks = [&](int rows) { return static_cast<long>(columns) * ((j.height + rows - 1) / rows); };
+  // A block of its own for every channel where blocks of all channels would
+  // leave the GPU (three resident per SM) short of a wave, although each then
+  // reads every cache line of the image.  All channels in a block against one:
+  // 640x480x3 K = 5 / 7 8.3 / 16.7 us against 5.7 / 12.3 us, 1024x768x3 (384 and
+  // 768 blocks) 14.2 / 31.9 against 13.2 / 30.1, 1280x720x3 (450 and 900) 14.1 /
+  // 32.3 against 14.6 / 33.8.  A block of K = 7 is half as wide, hence twice the
+  // count.
+  constexpr long kLayerBlocks = 1600 / median_width(K);
+  const int layers = blocks(4 * group) < kLayerBlocks ? j.channels : 1;
+  // Four warps on 4 groups of rows; fewer groups (all warps still stage) below
+  // one and a half such blocks per SM.  640x480x1 (150, 300 or 600 blocks of 16,
+  // 8 or 4 rows) K = 5: 16 rows 4.7 us, 8 rows 3.9 us, 4 rows 5.3 us.
   int rows = 4 * group;
-  while (rows > group && static_cast<long>(columns) * ((j.height + rows - 1) / rows) * j.channels < 304) rows /= 2;
+  while (rows > group && blocks(rows) * layers < 228) rows /= 2;
   const int row_blocks = (j.height + rows - 1) / rows;
-  // The smallest images also give every channel a block of its own.
-  const int layers = rows == group ? j.channels : 1;
   dim3 grid(static_cast<unsigned>(columns), static_cast<unsigned>(row_blocks < 65535 ? row_blocks : 65535),
             static_cast<unsigned>(layers));
   // At most 38,016 bytes (packed, four channels, K = 5).
