@@ -46,3 +46,25 @@ def test_unaligned_rows(dtype, w, h):
         assert pad_ok, n
         assert np.array_equal(got, want), (n, int((got != want).sum()))
     ctx.close()
+
+
+@pytest.mark.parametrize("dtype", ["u16", "s16"])
+@pytest.mark.parametrize("w,h", [(1023, 521), (1921, 700)])
+def test_unaligned_in_place(dtype, w, h):
+    """Source and destination are one unaligned image: every row is read as it was before the call."""
+    rng = np.random.default_rng(w * h + 1)
+    dt = np.dtype("uint16" if dtype == "u16" else "int16")
+    info = np.iinfo(dt)
+    kx, ky = TAPS[dtype]
+    ctx = kcv.Context.for_torch(0)
+    host = rng.integers(info.min, int(info.max) + 1, (h, w), dtype=dt)
+    buf, ptr, stride = device_image(torch, host, 2)
+    for _ in range(2):  # filtered twice
+        werr, want = oracle.separable_filter_2d(host, w, h, 1, np.array(kx, dt), np.array(ky, dt), kcv.REFLECT)
+        err = kcv.separable_filter_2d(dtype, ptr, stride, ptr, stride, w, h, 1, kx, 5, ky, 5, kcv.REFLECT, ctx)
+        assert err == werr == kcv.OK
+        assert ctx.synchronize() == kcv.OK
+        got, _ = read_output(buf, h, w, dt, stride, 2)
+        assert np.array_equal(got, want), int((got != want).sum())
+        host = want
+    ctx.close()

@@ -504,6 +504,14 @@ kleidicv_error_t resolve_context(kleidicv_gpu_context *&ctx) {
   return KLEIDICV_OK;
 }
 
+// Whether a destination of the same row bytes overlaps the source.
+static bool in_place(const FilterJob &f, size_t row) {
+  const uintptr_t s = reinterpret_cast<uintptr_t>(f.src), d = reinterpret_cast<uintptr_t>(f.dst);
+  const uintptr_t rows = static_cast<uintptr_t>(f.height) - 1;
+  return s < d + rows * static_cast<uintptr_t>(f.dst_stride) + row &&
+         d < s + rows * static_cast<uintptr_t>(f.src_stride) + row;
+}
+
 kleidicv_error_t execute(kleidicv_gpu_context *ctx, Prepared &p) {
   switch (p.kind) {
     case Prepared::NOTHING:
@@ -546,7 +554,26 @@ kleidicv_error_t execute(kleidicv_gpu_context *ctx, Prepared &p) {
       if (ctx->tune_threads <= 0 && sep16_eligible(p.fused)) {
         // One-channel 16-bit 5x5: the fp32 streaming kernel of sep16.cu.
         ctx->launches += 1;
-        return cuda_status(ctx, launch_sep16(p.fused, ctx->sm_count, ctx->stream));
+        // It reads rows while others are written.  A call in place on unaligned
+        // rows filters a pool image with 16-byte rows, while the pool has room.
+        const size_t row = static_cast<size_t>(p.fused.width) * 2, stride = (row + 15) / 16 * 16;
+        const size_t bytes = stride * p.fused.height;
+        uint8_t *image = nullptr;
+        if (((reinterpret_cast<uintptr_t>(p.fused.src) | static_cast<uintptr_t>(p.fused.src_stride)) & 15) != 0 &&
+            in_place(p.fused, row)) {
+          image = static_cast<uint8_t *>(ctx_alloc(ctx, bytes));
+        }
+        if (!image) return cuda_status(ctx, launch_sep16(p.fused, ctx->sm_count, ctx->stream));
+        cudaError_t e = cudaMemcpy2DAsync(image, stride, p.fused.src, p.fused.src_stride, row, p.fused.height,
+                                          cudaMemcpyDeviceToDevice, ctx->stream);
+        if (e == cudaSuccess) {
+          p.fused.src = image;
+          p.fused.src_stride = static_cast<int64_t>(stride);
+          e = launch_sep16(p.fused, ctx->sm_count, ctx->stream);
+        }
+        // Stream-ordered: the image is released after the filter has read it.
+        ctx_free(ctx, image, bytes);
+        return cuda_status(ctx, e);
       }
       if (ctx->tune_threads > 0) {
         TileShape t{ctx->tune_threads, ctx->tune_tile_rows, ctx->tune_stage_rows, ctx->tune_stages};
