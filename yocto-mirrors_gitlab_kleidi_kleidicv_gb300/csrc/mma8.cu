@@ -52,14 +52,15 @@ bool plan(Mma8Job &j, int sm_count) {
   j.nk = (8 + 2 * j.r + 15) / 16;
   j.nb = (j.vo + 16 + j.rc + 15) / 16;
   j.na = (j.vo + 8 + j.rc + 15) / 16;
-  // 64 x 256 bytes where that gives every SM two tiles, else 32 x 256:
-  // 3840x2160x1 7 taps 7.7 us against 8.4 us, 1920x1080x1 5.8 us against
-  // 4.7 us, 640x480x1 4.1 us against 3.6 us (16 x 128 gained nothing there;
-  // all with three CTAs per SM).
+  // Tiles of 32 rows x 256 bytes while two per SM, the resident CTAs, cover the
+  // image; else 64 rows, whose halo costs half.  32 against 64 rows, 9 taps:
+  // 1920x1200x1 (304 tiles of 32 rows, a full wave) 4.2 / 4.9 us, 2560x1080x1 (340)
+  // 5.2 / 5.0 us, 2560x1440x1 (450) 5.9 / 5.1 us, 1366x768x3 (408) 8.9 / 7.2 us.  The least gain is at
+  // 1280x720x3 (345): 5.5 / 5.4 us, and 6.5 / 6.7 us with 15 taps.
   j.tile_w = 256;
   for (j.mt = 4;; j.mt = 2) {
     if (!shape(j)) return false;
-    if (j.mt == 2 || !fixed_steps(j) || static_cast<long>(j.tiles_x) * j.tiles_y >= 2L * sm_count) return true;
+    if (j.mt == 2 || !fixed_steps(j) || static_cast<long>(j.tiles_x) * ((j.h + 31) / 32) > 2L * sm_count) return true;
   }
 }
 
