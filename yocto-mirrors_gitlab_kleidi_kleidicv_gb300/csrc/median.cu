@@ -167,8 +167,9 @@ __device__ __forceinline__ uint32_t med3(uint32_t a, uint32_t b, uint32_t c) {
 // median middle and the smallest maximum of the window's rows.  Packed: rows r
 // and r + 2 share a word, 12 minima and maxima per element (18 otherwise) where
 // selecting from each window took 42.  Measured: u8 1920x1080x1 14.4 -> 7.1 us,
-// 160x120x1 4.2 -> 3.8 us; f32 1280x720x3 18.6 -> 12.4 us (the kernel below, at
-// K = 3: 8.3, 6.3 and 20.5 us).  Bound by issue: 68 % of the slots and half of
+// 160x120x1 4.2 -> 3.8 us; f32 1280x720x3 18.6 -> 10.8 us (the kernel below, at
+// K = 3: 8.3, 6.3 and 20.5 us; non-coherent loads, which a source still being
+// written rules out, f32 10.0 us, 8 and 16 bits the same).  Bound by issue: 68 % of the slots and half of
 // the ALU pipe, 18 % of the load pipe, 74 % of the warps resident.
 template <typename T>
 __global__ void __launch_bounds__(128) median3_kernel(const uint8_t *src, int64_t src_stride, uint8_t *dst,
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(128) median3_kernel(const uint8_t *src, int64_
       const T *row = reinterpret_cast<const T *>(
           src + static_cast<int64_t>(map_index(y0 + r - 1, h, border)) * src_stride);
 #pragma unroll
-      for (int d = 0; d < 3; ++d) key[r][d] = Key<T>::to(__ldg(row + at[d]));
+      for (int d = 0; d < 3; ++d) key[r][d] = Key<T>::to(ld_src(row + at[d]));
     }
     uint32_t s[N][3];
 #pragma unroll
@@ -274,7 +275,7 @@ __device__ __forceinline__ void median_stage(uint32_t *stage, const uint8_t *src
         const int px = i / C;
         const int at = (inner ? x0 - R + px : map_index(x0 - R + px, w, border)) * (C > 1 ? C : c) + c0 + (i - px * C);
 #pragma unroll
-        for (int q = 0; q < kRows; ++q) v[q][k] = Key<T>::to(__ldg(r[q] + at));
+        for (int q = 0; q < kRows; ++q) v[q][k] = Key<T>::to(ld_src(r[q] + at));
       }
 #pragma unroll
       for (int k = 0; k < kAhead; ++k) {
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(kHistThreads) median_hist_kernel(const uint8_t
   const int m = (k * k - 1) / 2;  // rank of the median
   auto value = [&](int yy, int xx) -> int {
     const uint8_t *row = src + static_cast<int64_t>(map_index(yy, h, border)) * src_stride;
-    return __ldg(row + map_index(xx, w, border) * c + ch);
+    return row[map_index(xx, w, border) * c + ch];
   };
   // Rows loop over the grid's y extent, which the hardware caps at 65535.
   for (int y = blockIdx.y; y < h; y += gridDim.y) {

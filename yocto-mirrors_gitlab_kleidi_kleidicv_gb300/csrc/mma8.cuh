@@ -302,8 +302,8 @@ __device__ __forceinline__ void stage_pieces(const Mma8Job &j, uint8_t *raw, int
         const uint8_t *g = base + static_cast<int64_t>(y) * j.src_stride;
         const int m = static_cast<int>(reinterpret_cast<uintptr_t>(g) & 15);
         if (y >= 0 && g - m >= j.src && g - m + 32 <= end) {
-          u[k] = ld_nc_v4(g - m);
-          v[k] = ld_nc_v4(g - m + 16);
+          u[k] = ld_src_v4(g - m);
+          v[k] = ld_src_v4(g - m + 16);
           sh[k] = m;
         }
       }
@@ -318,7 +318,7 @@ __device__ __forceinline__ void stage_pieces(const Mma8Job &j, uint8_t *raw, int
             *reinterpret_cast<uint4 *>(d) = make_uint4(bv, bv, bv, bv);
           } else {
             const uint8_t *g = base + static_cast<int64_t>(y) * j.src_stride;
-            for (int i = 0; i < min(16, avail); ++i) d[i] = __ldg(g + i);
+            for (int i = 0; i < min(16, avail); ++i) d[i] = ld_src(g + i);
           }
         }
       }
@@ -369,7 +369,7 @@ __device__ __forceinline__ void fill_border_columns(const Mma8Job &j, uint8_t *r
         v = raw[row * pitch + from - xb];
       } else if (from >= 0) {
         const int y = map_index(y0 + row, j.h, j.border);
-        if (y >= 0) v = __ldg(j.src + static_cast<int64_t>(y) * j.src_stride + from);
+        if (y >= 0) v = ld_src(j.src + static_cast<int64_t>(y) * j.src_stride + from);
       }
       raw[row * pitch + x - xb] = v;
     }

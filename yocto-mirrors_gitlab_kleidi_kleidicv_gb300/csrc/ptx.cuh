@@ -130,9 +130,23 @@ __device__ __forceinline__ int32_t add_sat_s32(int32_t a, int32_t b) {
   return d;
 }
 
-__device__ __forceinline__ uint4 ld_nc_v4(const void *p) {
+// Loads of source images.  The kernels that use them are launched early: their
+// CTAs are resident while the call before may still write the source, so the
+// source is not read-only for the kernel's lifetime and the non-coherent loads
+// (__ldg, ld.global.nc) may not be used on it.  grid_dependency_wait orders
+// these (volatile: they stay behind it).
+template <typename T>
+__device__ __forceinline__ T ld_src(const T *p) {
+  uint32_t v;
+  if constexpr (sizeof(T) == 1) asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p));
+  else if constexpr (sizeof(T) == 2) asm volatile("ld.global.u16 %0, [%1];" : "=r"(v) : "l"(p));
+  else asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  if constexpr (sizeof(T) == 4) return *reinterpret_cast<const T *>(&v);
+  else return static_cast<T>(v);
+}
+__device__ __forceinline__ uint4 ld_src_v4(const void *p) {
   uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;

@@ -368,7 +368,7 @@ __device__ __forceinline__ void edge_task(const PyrEntry &e, int task) {
 #pragma unroll
   for (int r = 0; r < 5; ++r)
 #pragma unroll
-    for (int c = 0; c < 5; ++c) v[r][c] = (rows[r] && cols[c] >= 0) ? __ldg(rows[r] + cols[c]) : bv;
+    for (int c = 0; c < 5; ++c) v[r][c] = (rows[r] && cols[c] >= 0) ? ld_src(rows[r] + cols[c]) : bv;
   const uint32_t wt[5] = {1, 4, 6, 4, 1};
   uint32_t sum = 128;
 #pragma unroll

@@ -189,7 +189,7 @@ __device__ __forceinline__ void edge_element16(const Sep16Job &j, int y, int x) 
 #pragma unroll
   for (int r = 0; r < 5; ++r)
 #pragma unroll
-    for (int c = 0; c < 5; ++c) raw[r][c] = (rows[r] && cols[c] >= 0) ? __ldg(rows[r] + cols[c]) : bv;
+    for (int c = 0; c < 5; ++c) raw[r][c] = (rows[r] && cols[c] >= 0) ? ld_src(rows[r] + cols[c]) : bv;
   float2 kx[5];
 #pragma unroll
   for (int t = 0; t < 5; ++t) kx[t] = make_float2(j.kx[t], j.kx[t]);
@@ -242,7 +242,7 @@ __device__ __forceinline__ void stage_block16(const Sep16Job &j, uint4 *slot, in
   } else {
     uint16_t *d = reinterpret_cast<uint16_t *>(slot);
     for (int k = static_cast<int>(j.src - a) / 2; k < 8; ++k)
-      d[k] = 2 * k < left ? __ldg(reinterpret_cast<const uint16_t *>(a) + k) : uint16_t{0};
+      d[k] = 2 * k < left ? ld_src(reinterpret_cast<const uint16_t *>(a) + k) : uint16_t{0};
   }
 }
 

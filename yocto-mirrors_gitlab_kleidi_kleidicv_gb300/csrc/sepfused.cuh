@@ -113,12 +113,12 @@ __device__ __forceinline__ bool load_chunk_fast(const uint8_t *row, long xb, lon
   const uint8_t *p = row + xb;
   const uintptr_t pa = reinterpret_cast<uintptr_t>(p);
   if ((pa & 15) == 0) {
-    out = ld_nc_v4(p);
+    out = ld_src_v4(p);
     return true;
   }
   const uint8_t *a = reinterpret_cast<const uint8_t *>(pa & ~static_cast<uintptr_t>(15));
   if (a < row || a + 32 > row + wcb) return false;
-  const uint4 u = ld_nc_v4(a), v = ld_nc_v4(a + 16);
+  const uint4 u = ld_src_v4(a), v = ld_src_v4(a + 16);
   out = shift_blocks(u, v, static_cast<int>(pa & 15));
   return true;
 }
@@ -1067,7 +1067,7 @@ __device__ __forceinline__ void run_tile(const FilterJob &j, const TmaMaps &maps
         } else {
           const uint8_t *grow =
               j.src + static_cast<int64_t>(map_index(iy, j.height, j.border)) * j.src_stride;
-          v = ES == 1 ? __ldg(grow + me) : __ldg(reinterpret_cast<const uint16_t *>(grow) + me);
+          v = ES == 1 ? ld_src(grow + me) : ld_src(reinterpret_cast<const uint16_t *>(grow) + me);
         }
         uint8_t *dst = lbase + rr * lpitch + e * ES;
         dst[0] = static_cast<uint8_t>(v);

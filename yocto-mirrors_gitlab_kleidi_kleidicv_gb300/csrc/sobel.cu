@@ -45,7 +45,7 @@ __device__ __forceinline__ void load_window(const SobelJob &j, const uint8_t *ro
     const int sh = static_cast<int>(a & 3) * 8;
     uint32_t w[NW + 1];
 #pragma unroll
-    for (int k = 0; k <= NW; ++k) w[k] = __ldg(p + k);
+    for (int k = 0; k <= NW; ++k) w[k] = ld_src(p + k);
 #pragma unroll
     for (int k = 0; k < NW; ++k) {
       const uint32_t v = __funnelshift_r(w[k], w[k + 1], sh);
@@ -58,7 +58,7 @@ __device__ __forceinline__ void load_window(const SobelJob &j, const uint8_t *ro
     for (int i = 0; i < N; ++i) {
       const int e = e0 - C + i, ch = (e + 4 * C) % C;  // e >= -C
       const int lo = max(e, ch), hi = j.wc - C + ch;     // the first and last pixel's element
-      x[i] = __ldg(row + min(lo, hi));
+      x[i] = ld_src(row + min(lo, hi));
     }
   }
 }
