@@ -5,6 +5,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <numeric>
 #include <mutex>
 
@@ -504,12 +505,27 @@ kleidicv_error_t resolve_context(kleidicv_gpu_context *&ctx) {
   return KLEIDICV_OK;
 }
 
-// Whether a destination of the same row bytes overlaps the source.
+// Whether a destination row shares a byte with a source row (`row` bytes each).
+// Images may share a buffer without that: side by side, or row by row.
 static bool in_place(const FilterJob &f, size_t row) {
-  const uintptr_t s = reinterpret_cast<uintptr_t>(f.src), d = reinterpret_cast<uintptr_t>(f.dst);
-  const uintptr_t rows = static_cast<uintptr_t>(f.height) - 1;
-  return s < d + rows * static_cast<uintptr_t>(f.dst_stride) + row &&
-         d < s + rows * static_cast<uintptr_t>(f.src_stride) + row;
+  const int64_t n = static_cast<int64_t>(row), h = f.height, ss = f.src_stride, ds = f.dst_stride;
+  // The first destination row lies `o` bytes past the first source row.
+  const int64_t o = static_cast<int64_t>(reinterpret_cast<uintptr_t>(f.dst) - reinterpret_cast<uintptr_t>(f.src));
+  if (o >= (h - 1) * ss + n || -o >= (h - 1) * ds + n) return false;
+  if (h == 1 || ss < n || ds < n) return true;
+  if (ss == ds) {
+    // o = q ss + m: destination row y starts m bytes into source row y + q.
+    const int64_t q = o >= 0 ? o / ss : -((-o + ss - 1) / ss), m = o - q * ss;
+    return (m < n && std::abs(q) < h) || (ss - m < n && std::abs(q + 1) < h);
+  }
+  // Both in ascending order: the row that ends first cannot meet a later one.
+  for (int64_t sy = 0, dy = 0; sy < h && dy < h;) {
+    const int64_t s0 = sy * ss, d0 = o + dy * ds;
+    if (s0 < d0 + n && d0 < s0 + n) return true;
+    if (s0 < d0) ++sy;
+    else ++dy;
+  }
+  return false;
 }
 
 kleidicv_error_t execute(kleidicv_gpu_context *ctx, Prepared &p) {
