@@ -77,3 +77,32 @@ def test_images_that_share_no_byte(dtype, w, h, layout):
     assert np.array_equal(got, host), int((got != host).sum())
     assert _arbitrary(ctx) == kcv.ALLOCATION  # the failure is still to come
     ctx.close()
+
+
+@pytest.mark.parametrize("dtype", ["u16", "s16"])
+@pytest.mark.parametrize("w,h", [(151, 47), (1023, 521)])
+def test_in_place_without_room_is_refused(dtype, w, h):
+    """A call in place needs a copy of its source: without one it is refused and
+    the image stays as it is."""
+    rng = np.random.default_rng(w)
+    dt = np.dtype("uint16" if dtype == "u16" else "int16")
+    info = np.iinfo(dt)
+    host = rng.integers(info.min, int(info.max) + 1, (h, w), dtype=dt)
+    buf, ptr, stride = device_image(torch, host, 2)
+
+    def image():
+        return buf.cpu().numpy()[2:2 + host.nbytes].view(dt).reshape(h, w)
+
+    capped = kcv.Context(0, torch.cuda.current_stream().cuda_stream, pool_limit=1024)
+    assert _call(dtype, ptr, stride, ptr, stride, w, h, capped) == kcv.ALLOCATION
+    assert capped.synchronize() == kcv.OK
+    capped.close()
+    ctx = kcv.Context.for_torch(0)
+    ctx.fail_next_allocations(1)
+    assert _call(dtype, ptr, stride, ptr, stride, w, h, ctx) == kcv.ALLOCATION
+    assert ctx.synchronize() == kcv.OK
+    assert np.array_equal(image(), host)
+    assert _call(dtype, ptr, stride, ptr, stride, w, h, ctx) == kcv.OK
+    assert ctx.synchronize() == kcv.OK
+    assert np.array_equal(image(), _want(dtype, host, w, h))
+    ctx.close()

@@ -569,17 +569,19 @@ kleidicv_error_t execute(kleidicv_gpu_context *ctx, Prepared &p) {
       }
       if (ctx->tune_threads <= 0 && sep16_eligible(p.fused)) {
         // One-channel 16-bit 5x5: the fp32 streaming kernel of sep16.cu.
-        ctx->launches += 1;
-        // It reads rows while others are written.  A call in place on unaligned
-        // rows filters a pool image with 16-byte rows, while the pool has room.
+        // It reads rows while others are written: a call in place on unaligned
+        // rows filters a pool image with 16-byte rows, and is refused where the
+        // pool has no room for one (no kernel here can answer it then).
         const size_t row = static_cast<size_t>(p.fused.width) * 2, stride = (row + 15) / 16 * 16;
         const size_t bytes = stride * p.fused.height;
-        uint8_t *image = nullptr;
-        if (((reinterpret_cast<uintptr_t>(p.fused.src) | static_cast<uintptr_t>(p.fused.src_stride)) & 15) != 0 &&
-            in_place(p.fused, row)) {
-          image = static_cast<uint8_t *>(ctx_alloc(ctx, bytes));
+        if (((reinterpret_cast<uintptr_t>(p.fused.src) | static_cast<uintptr_t>(p.fused.src_stride)) & 15) == 0 ||
+            !in_place(p.fused, row)) {
+          ctx->launches += 1;
+          return cuda_status(ctx, launch_sep16(p.fused, ctx->sm_count, ctx->stream));
         }
-        if (!image) return cuda_status(ctx, launch_sep16(p.fused, ctx->sm_count, ctx->stream));
+        uint8_t *image = static_cast<uint8_t *>(ctx_alloc(ctx, bytes));
+        if (!image) return KLEIDICV_ERROR_ALLOCATION;
+        ctx->launches += 1;
         cudaError_t e = cudaMemcpy2DAsync(image, stride, p.fused.src, p.fused.src_stride, row, p.fused.height,
                                           cudaMemcpyDeviceToDevice, ctx->stream);
         if (e == cudaSuccess) {
