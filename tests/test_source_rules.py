@@ -25,3 +25,13 @@ def test_kernels_launched_early_use_no_non_coherent_loads():
     early = [n for n, s in sources.items() if n.endswith(".cuh") or "grid_dependency_wait" in s]
     assert len(early) > 5
     assert [n for n in early if re.search(r"__ldg\s*\(|ld\.global\.nc", sources[n])] == []
+
+
+def test_asynchronous_copies_are_ordered_for_the_compiler():
+    """A copy into a staged slot that is read and refilled: without a "memory"
+    clobber the compiler may move the read behind the copy."""
+    copies = []
+    for name, s in _sources().items():
+        copies += [(name, m) for m in re.findall(r'asm volatile\(\s*"cp\.async\.c[ag][^;]*;.*?\);', s, flags=re.S)]
+    assert len(copies) >= 6
+    assert [c for c in copies if '"memory"' not in c[1]] == []

@@ -55,8 +55,9 @@ constexpr int ring_groups(int k) { return k == 3 ? 3 : k == 5 ? 4 : 2; }
 constexpr int warp_stage8(int k) { return ring_groups(k) * k * 32 * 16; }  // bytes
 constexpr int smem8(int k) { return kWarpsG * warp_stage8(k); }
 
+// The "memory" clobbers keep earlier reads of a ring slot ahead of its copies.
 __device__ __forceinline__ void cp_async16g(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit_g() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -154,7 +155,7 @@ __device__ __forceinline__ uint4 filter_row8(const uint32_t (&wl)[K][kPix], cons
 }
 
 __device__ __forceinline__ void cp_async4g(uint32_t dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 
 template <int K, bool SIMPLE, typename Copy>
@@ -278,7 +279,10 @@ __device__ __forceinline__ void band_loop8(const Gauss8Job &j, const uint4 *stag
       if (base + S >= rows) return;  // past the band (the loop ends here)
       unpack4(S == 0 ? cur[(K - 1) * 32] : next[(S - 1) * 32], wl[slot], wh[slot]);
       if constexpr (S == 0)
-        if (G::kRing) copy_group(grp + G::kGroups);
+        if (G::kRing) {
+          __syncwarp();  // every lane has read the last row of group grp
+          copy_group(grp + G::kGroups);
+        }
       const uint4 out = filter_row8<K, S>(wl, wh, wt);
       if (SIMPLE) {
         if (outputs) *reinterpret_cast<uint4 *>(d) = out;

@@ -97,9 +97,9 @@ __host__ __device__ constexpr uint32_t tap_word(int c, int j, int q) {
   return w;
 }
 
-// No "memory" clobber: nothing reads the slot before the wait.
+// The "memory" clobber keeps earlier reads of the slot ahead of it.
 __device__ __forceinline__ void cp_async16p(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit_p() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>

@@ -74,10 +74,9 @@ constexpr int warp_stage16(bool aligned) { return kStageRows * slots16(aligned);
 constexpr int smem16(bool aligned) { return kWarps16 * warp_stage16(aligned) * 16; }  // 38912, 40128
 constexpr int kGroups = (kStageRows + 4) / 5;          // copy groups of five rows: 4
 
-// No "memory" clobber: nothing reads the slot before cp_async_wait, which
-// carries it.
+// The "memory" clobber keeps the last band's reads of the slot ahead of it.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -238,7 +237,8 @@ __device__ __forceinline__ void stage_block16(const Sep16Job &j, uint4 *slot, in
     const int n = left >= 16 ? 16 : left > 0 ? static_cast<int>(left) : 0;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
                      static_cast<uint32_t>(__cvta_generic_to_shared(slot))),
-                 "l"(n > 0 ? a : a - 16), "r"(n));
+                 "l"(n > 0 ? a : a - 16), "r"(n)
+                 : "memory");
   } else {
     uint16_t *d = reinterpret_cast<uint16_t *>(slot);
     for (int k = static_cast<int>(j.src - a) / 2; k < 8; ++k)
@@ -483,7 +483,7 @@ __device__ __forceinline__ void band_loop16(const Sep16Job &j, const uint4 *stag
       d += j.dst_stride;
     });
   }
-  if (!ALIGNED) __syncwarp();  // the next item's copies may overwrite the slots
+  __syncwarp();  // the next item's copies may overwrite the slots
 }
 
 template <bool S16, bool ALIGNED>
