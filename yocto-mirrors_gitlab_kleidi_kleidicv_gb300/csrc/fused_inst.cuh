@@ -32,6 +32,43 @@ cudaError_t allow_large_smem() {
   return e;
 }
 
+// A plain launch (launch_one) of the kernel compiled for LOADS.
+template <int MODE, int K, int C, bool NARROW, int LOADS>
+cudaError_t launch_single(const FilterJob &job, int *err_flag, cudaStream_t stream, int *blocks_per_sm) {
+  const SmemLayout L = smem_layout(MODE, K, C, job.threads, job.halo_chunks, job.box_lbw,
+                                   job.stage_rows, job.stages, job.use_tma != 0,
+                                   job.border == BORDER_WRAP);
+  auto kern = sepfused_kernel<MODE, K, C, NARROW, LOADS>;
+  if (cudaError_t e = allow_large_smem<sepfused_kernel<MODE, K, C, NARROW, LOADS>>(); e != cudaSuccess)
+    return e;
+  // One wave of persistent CTAs: as many as fit on the device at once.
+  int per_sm = 0, dev = 0, sms = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, job.threads, L.total);
+  if (e != cudaSuccess) return e;
+  if (blocks_per_sm) {
+    *blocks_per_sm = per_sm;
+    return cudaSuccess;
+  }
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long tiles = static_cast<long>(job.strips) * job.row_tiles;
+  const long grid = std::max(1L, std::min(tiles, static_cast<long>(std::max(per_sm, 1)) * sms));
+  // Programmatic stream serialization: this launch may begin while the
+  // previous kernel on the stream drains (the kernel waits for it before
+  // touching memory).
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(job.threads));
+  cfg.dynamicSmemBytes = L.total;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, job, err_flag);
+}
+
 // Plain launch of `job` (batch == nullptr) or of the batched kernel of the
 // same instantiation over batch->tiles.  With blocks_per_sm set, only reports
 // the occupancy.
@@ -64,38 +101,11 @@ cudaError_t launch_one(const FilterJob &job, int *err_flag, cudaStream_t stream,
         batch->jobs, batch->tiles, batch->ntiles, batch->next_tile, err_flag);
     return cudaGetLastError();
   }
-  const SmemLayout L = smem_layout(MODE, K, C, job.threads, job.halo_chunks, job.box_lbw,
-                                   job.stage_rows, job.stages, job.use_tma != 0,
-                                   job.border == BORDER_WRAP);
-  auto kern = sepfused_kernel<MODE, K, C, NARROW>;
-  if (cudaError_t e = allow_large_smem<sepfused_kernel<MODE, K, C, NARROW>>(); e != cudaSuccess)
-    return e;
-  // One wave of persistent CTAs: as many as fit on the device at once.
-  int per_sm = 0, dev = 0, sms = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, job.threads, L.total);
-  if (e != cudaSuccess) return e;
-  if (blocks_per_sm) {
-    *blocks_per_sm = per_sm;
-    return cudaSuccess;
-  }
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long tiles = static_cast<long>(job.strips) * job.row_tiles;
-  const long grid = std::max(1L, std::min(tiles, static_cast<long>(std::max(per_sm, 1)) * sms));
-  // Programmatic stream serialization: this launch may begin while the
-  // previous kernel on the stream drains (the kernel waits for it before
-  // touching memory).
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid));
-  cfg.blockDim = dim3(static_cast<unsigned>(job.threads));
-  cfg.dynamicSmemBytes = L.total;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, job, err_flag);
+  if constexpr (MODE == MODE_BINOM)
+    return job.use_tma ? launch_single<MODE, K, C, NARROW, kLoadsTma>(job, err_flag, stream, blocks_per_sm)
+                       : launch_single<MODE, K, C, NARROW, kLoadsPlain>(job, err_flag, stream, blocks_per_sm);
+  else
+    return launch_single<MODE, K, C, NARROW, kLoadsByJob>(job, err_flag, stream, blocks_per_sm);
 }
 
 template <int MODE, int K, bool NARROW>

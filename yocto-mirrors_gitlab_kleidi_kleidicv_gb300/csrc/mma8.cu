@@ -95,7 +95,7 @@ bool mma8_job(const FilterJob &f, int sm_count, Mma8Job &j) {
   // The binomial 3x3 and 5x5 need two planes of vertical results here, and the
   // tiled stencil has cheap (constant) taps for them: it keeps the larger
   // images whose rows TMA can load.  5x5, tiled against here: 320x240x1 8.5 /
-  // 3.9 us, 1920x1080x1 7.0 / 4.5 us, 1920x1080x3 9.6 / 9.9 us, 3840x2160x3 19.2
+  // 3.9 us, 1920x1080x1 7.0 / 4.5 us, 1920x1080x3 9.3 / 9.9 us, 3840x2160x3 18.8
   // / 23.3 us; unaligned rows 3841x2160x1 26.3 / 14.5 us, x4 60.3 / 43.9 us.
   const bool unaligned = ((reinterpret_cast<uintptr_t>(f.src) | static_cast<uintptr_t>(f.src_stride)) & 15) != 0;
   const bool binomial = f.mode == MODE_BINOM && f.ksize <= 5 &&

@@ -764,8 +764,10 @@ struct TmaMaps {
 // stages used by this CTA so far (mbarrier phases continue across tiles).
 // stage_rows and stages are powers of two.  SHIFT_STORES compiles the
 // aligned-block stores for destination rows that are not 16-byte aligned
-// (store_shifted); without it such rows are written byte by byte.
-template <int MODE, int K, int C, bool NARROW, bool SHIFT_STORES>
+// (store_shifted); without it such rows are written byte by byte.  LOADS says
+// how rows are staged where the kernel is compiled for one way.
+enum TileLoads { kLoadsByJob, kLoadsTma, kLoadsPlain };
+template <int MODE, int K, int C, bool NARROW, bool SHIFT_STORES, int LOADS = kLoadsByJob>
 __device__ __forceinline__ void run_tile(const FilterJob &j, const TmaMaps &maps, int strip,
                                          int band, uint8_t *smem, uint32_t &gstage,
                                          int *err_flag, bool &timed_out) {
@@ -780,7 +782,7 @@ __device__ __forceinline__ void run_tile(const FilterJob &j, const TmaMaps &maps
   const CtaShape sh = cta_shape(blockDim.x, HC, lbw);
   const int rb = j.stage_rows, ns = j.stages;
   const int lrb = __ffs(rb) - 1;
-  const bool use_tma = j.use_tma != 0;
+  const bool use_tma = LOADS == kLoadsByJob ? j.use_tma != 0 : LOADS == kLoadsTma;
   const SmemLayout L = smem_layout(MODE, K, C, blockDim.x, HC, lbw, rb, ns, use_tma,
                                    j.border == BORDER_WRAP);
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);
@@ -1223,14 +1225,18 @@ __device__ __forceinline__ void run_tile(const FilterJob &j, const TmaMaps &maps
 // Register budget: 4 resident CTAs per SM (2 for the 15/21 sizes).  Cutting
 // it for 5 (96 registers, which the shuffle modes fit without spilling) was
 // measured 7-11 % slower on 3840x2160 calls.
-template <int MODE, int K, int C, bool NARROW>
+// LOADS: the binomials have a kernel each for TMA and for plain loads.  In one
+// kernel for both, the code of either changed the speed of the other.  One / two:
+// 3840x2160x4 5x5 24.5 / 22.1 us, 9x9 59.2 / 53.0 us, x3 9x9 48.2 / 44.1 us, x4
+// 7x7 51.7 / 51.6 us; unaligned 3841x2160x1 7x7 38.9 / 33.8 us, x4 9x9 112 / 99 us.
+template <int MODE, int K, int C, bool NARROW, int LOADS>
 __global__ void __launch_bounds__(128, (K >= 15 ? 2 : 4))
     sepfused_kernel(const __grid_constant__ FilterJob job, int *err_flag) {
   extern __shared__ __align__(128) uint8_t smem[];
   // The next call on the stream may start its CTAs as ours finish (they only
   // fit where ours left room); everything it reads waits for our completion.
   launch_dependents();
-  if (job.use_tma) {
+  if (LOADS == kLoadsByJob ? job.use_tma != 0 : LOADS == kLoadsTma) {
     if (threadIdx.x == 0) {
       prefetch_tensormap(&job.tmap);
       prefetch_tensormap(&job.tmap_row);
@@ -1252,8 +1258,8 @@ __global__ void __launch_bounds__(128, (K >= 15 ? 2 : 4))
   // above overlapped its tail).
   grid_dependency_wait();
   for (int t = blockIdx.x; t < tiles; t += gridDim.x)
-    run_tile<MODE, K, C, NARROW, true>(job, maps, t % job.strips, t / job.strips, smem, gstage,
-                                 err_flag, timed_out);
+    run_tile<MODE, K, C, NARROW, true, LOADS>(job, maps, t % job.strips, t / job.strips, smem, gstage, err_flag,
+                                              timed_out);
 }
 
 }  // namespace kcv
