@@ -443,7 +443,9 @@ kleidicv_error_t cuda_status(kleidicv_gpu_context *ctx, cudaError_t e) {
   return KLEIDICV_GPU_ERROR_CUDA;
 }
 
-cudaError_t upload_async(kleidicv_gpu_context *ctx, void *dst, const void *src, size_t bytes) {
+cudaError_t upload_async(kleidicv_gpu_context *ctx, void *dst, const UploadPiece *pieces, size_t n) {
+  size_t bytes = 0;
+  for (size_t k = 0; k < n; ++k) bytes = std::max(bytes, pieces[k].at + pieces[k].bytes);
   if (bytes == 0) return cudaSuccess;
   std::lock_guard<std::mutex> lock(ctx->upload_mutex);
   kleidicv_gpu_context::UploadSlot &u = ctx->upload[ctx->upload_next];
@@ -461,10 +463,16 @@ cudaError_t upload_async(kleidicv_gpu_context *ctx, void *dst, const void *src, 
     }
     u.bytes = bytes;
   }
-  memcpy(u.host, src, bytes);
+  for (size_t k = 0; k < n; ++k)
+    if (pieces[k].bytes) memcpy(static_cast<uint8_t *>(u.host) + pieces[k].at, pieces[k].src, pieces[k].bytes);
   e = cudaMemcpyAsync(dst, u.host, bytes, cudaMemcpyHostToDevice, ctx->stream);
   if (e != cudaSuccess) return e;
   return cudaEventRecord(u.done, ctx->stream);
+}
+
+cudaError_t upload_async(kleidicv_gpu_context *ctx, void *dst, const void *src, size_t bytes) {
+  const UploadPiece piece{0, src, bytes};
+  return upload_async(ctx, dst, &piece, 1);
 }
 
 bool ctx_admits(kleidicv_gpu_context *ctx, size_t bytes) {

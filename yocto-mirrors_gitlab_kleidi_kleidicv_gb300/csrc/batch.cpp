@@ -328,7 +328,7 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
     }
   }
 
-  // Largest tiles first within each group; device layout [jobs][tiles][counters][scratch].
+  // Largest tiles first within each group.
   std::vector<BatchTile> all_tiles;
   for (Group &gr : p->groups) {
     std::vector<size_t> order(gr.tiles.size());
@@ -347,7 +347,7 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
   p->tiles_total = all_tiles.size();
   // Blur-and-downsample entries: bands sized for each request's share of the
   // pyramid kernel's resident warps, items counted through the table.
-  size_t npyr_groups = 0, pyr_bytes[4] = {0, 0, 0, 0};
+  size_t npyr_groups = 0;
   for (int c = 0; c < 4; ++c) {
     std::vector<PyrEntry> &v = p->pyr[c];
     if (v.empty()) continue;
@@ -360,11 +360,10 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
       items += en.item_end;
       en.item_end = items;
     }
-    pyr_bytes[c] = align_up(v.size() * sizeof(PyrEntry), 256);
   }
   // Four-channel Gaussians: bands sized for each request's share of the
   // streaming kernel's resident warps, items counted through the table.
-  size_t ng8_groups = 0, g8_bytes[3] = {0, 0, 0};
+  size_t ng8_groups = 0;
   for (int k = 0; k < 3; ++k) {
     std::vector<Gauss8Job> &v = p->g8[k];
     if (v.empty()) continue;
@@ -376,20 +375,31 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
       items += g.strips * g.bands;
       g.item_end = items;
     }
-    g8_bytes[k] = align_up(v.size() * sizeof(Gauss8Job), 256);
   }
-  const size_t jobs_bytes = align_up(p->jobs.size() * sizeof(FilterJob), 256);
-  const size_t tiles_bytes = align_up(all_tiles.size() * sizeof(BatchTile), 256);
-  const size_t next_bytes = align_up(p->groups.size() * sizeof(int), 256);
-  const size_t pyr_total = pyr_bytes[0] + pyr_bytes[1] + pyr_bytes[2] + pyr_bytes[3];
-  const size_t g8_total = g8_bytes[0] + g8_bytes[1] + g8_bytes[2];
-  size_t mma8_total = p->mma8.empty() ? 0 : align_up(p->mma8.size() * sizeof(int), 256);
+  // The tables, which go up in one piece; the counters; the scratch images.
+  size_t end = 0;
+  const auto place = [&end](size_t bytes) {
+    const size_t at = end;
+    end += align_up(bytes, 256);
+    return at;
+  };
+  std::vector<UploadPiece> tables;
+  const auto add = [&](const auto &v) {
+    tables.push_back(UploadPiece{place(v.size() * sizeof(v[0])), v.data(), v.size() * sizeof(v[0])});
+    return tables.back().at;
+  };
+  const size_t jobs_at = add(p->jobs), tiles_at = add(all_tiles);
+  size_t pyr_at[4], g8_at[3];
+  for (int c = 0; c < 4; ++c) pyr_at[c] = add(p->pyr[c]);
+  for (int k = 0; k < 3; ++k) g8_at[k] = add(p->g8[k]);
+  std::vector<size_t> mma8_at;
   for (auto &m : p->mma8) {
-    mma8_total += align_up(m.second.jobs.size() * sizeof(Mma8Job), 256) +
-                  align_up(m.second.ends.size() * sizeof(int), 256);
+    mma8_at.push_back(add(m.second.jobs));
+    mma8_at.push_back(add(m.second.ends));
     p->tiles_total += m.second.tiles;
   }
-  p->dmem_bytes = jobs_bytes + tiles_bytes + next_bytes + generic_bytes + pyr_total + g8_total + mma8_total;
+  const size_t next_at = place(p->groups.size() * sizeof(int)), mma8_next_at = place(p->mma8.size() * sizeof(int));
+  p->dmem_bytes = end + generic_bytes;
   if (admitted_bytes && ctx->pool_used.load() + p->dmem_bytes + admitted_bytes > ctx->pool_limit) {
     delete p;
     return KLEIDICV_ERROR_ALLOCATION;
@@ -402,52 +412,27 @@ kleidicv_error_t kleidicv_gpu_batch_plan_create(const kleidicv_gpu_request_t *re
       return KLEIDICV_ERROR_ALLOCATION;
     }
   }
-  p->d_jobs = reinterpret_cast<FilterJob *>(p->dmem);
-  p->d_tiles = reinterpret_cast<BatchTile *>(p->dmem + jobs_bytes);
-  p->d_next = reinterpret_cast<int *>(p->dmem + jobs_bytes + tiles_bytes);
-  for (size_t &off : p->generic_off) off += jobs_bytes + tiles_bytes + next_bytes;
-  {
-    size_t off = jobs_bytes + tiles_bytes + next_bytes + generic_bytes;
-    for (int c = 0; c < 4; ++c) {
-      if (!pyr_bytes[c]) continue;
-      p->d_pyr[c] = reinterpret_cast<PyrEntry *>(p->dmem + off);
-      off += pyr_bytes[c];
-    }
-    for (int k = 0; k < 3; ++k) {
-      if (!g8_bytes[k]) continue;
-      p->d_g8[k] = reinterpret_cast<Gauss8Job *>(p->dmem + off);
-      off += g8_bytes[k];
-    }
-    // The counters, then each group's jobs and tile ends.
-    p->d_mma8_next = reinterpret_cast<int *>(p->dmem + off);
-    if (!p->mma8.empty()) off += align_up(p->mma8.size() * sizeof(int), 256);
-    int k = 0;
-    for (auto &m : p->mma8) {
-      Mma8Batch &b = m.second.batch;
-      b.jobs = reinterpret_cast<const Mma8Job *>(p->dmem + off);
-      off += align_up(m.second.jobs.size() * sizeof(Mma8Job), 256);
-      b.ends = reinterpret_cast<const int *>(p->dmem + off);
-      off += align_up(m.second.ends.size() * sizeof(int), 256);
-      b.n = static_cast<int>(m.second.jobs.size());
-      b.tiles = static_cast<int>(m.second.tiles);
-      b.next = p->d_mma8_next + k++;
-      b.smem_bytes = m.second.jobs[0].smem_bytes;  // of the instantiation
-    }
+  p->d_jobs = reinterpret_cast<FilterJob *>(p->dmem + jobs_at);
+  p->d_tiles = reinterpret_cast<BatchTile *>(p->dmem + tiles_at);
+  p->d_next = reinterpret_cast<int *>(p->dmem + next_at);
+  p->d_mma8_next = reinterpret_cast<int *>(p->dmem + mma8_next_at);
+  for (size_t &off : p->generic_off) off += end;
+  for (int c = 0; c < 4; ++c)
+    if (!p->pyr[c].empty()) p->d_pyr[c] = reinterpret_cast<PyrEntry *>(p->dmem + pyr_at[c]);
+  for (int k = 0; k < 3; ++k)
+    if (!p->g8[k].empty()) p->d_g8[k] = reinterpret_cast<Gauss8Job *>(p->dmem + g8_at[k]);
+  int group = 0;
+  for (auto &m : p->mma8) {
+    Mma8Batch &b = m.second.batch;
+    b.jobs = reinterpret_cast<const Mma8Job *>(p->dmem + mma8_at[2 * group]);
+    b.ends = reinterpret_cast<const int *>(p->dmem + mma8_at[2 * group + 1]);
+    b.n = static_cast<int>(m.second.jobs.size());
+    b.tiles = static_cast<int>(m.second.tiles);
+    b.next = p->d_mma8_next + group++;
+    b.smem_bytes = m.second.jobs[0].smem_bytes;  // of the instantiation
   }
   // Through the pinned upload ring: no wait for the stream's earlier work.
-  cudaError_t ce = upload_async(ctx, p->d_jobs, p->jobs.data(), p->jobs.size() * sizeof(FilterJob));
-  if (ce == cudaSuccess)
-    ce = upload_async(ctx, p->d_tiles, all_tiles.data(), all_tiles.size() * sizeof(BatchTile));
-  for (int c = 0; c < 4 && ce == cudaSuccess; ++c)
-    if (p->d_pyr[c]) ce = upload_async(ctx, p->d_pyr[c], p->pyr[c].data(), p->pyr[c].size() * sizeof(PyrEntry));
-  for (int k = 0; k < 3 && ce == cudaSuccess; ++k)
-    if (p->d_g8[k]) ce = upload_async(ctx, p->d_g8[k], p->g8[k].data(), p->g8[k].size() * sizeof(Gauss8Job));
-  for (auto &m : p->mma8) {
-    const Mma8Batch &b = m.second.batch;
-    if (ce == cudaSuccess)
-      ce = upload_async(ctx, const_cast<Mma8Job *>(b.jobs), m.second.jobs.data(), b.n * sizeof(Mma8Job));
-    if (ce == cudaSuccess) ce = upload_async(ctx, const_cast<int *>(b.ends), m.second.ends.data(), b.n * sizeof(int));
-  }
+  cudaError_t ce = upload_async(ctx, p->dmem, tables.data(), tables.size());
   const size_t nbranch = std::min<size_t>(kMaxBranches, p->groups.size() + npyr_groups + ng8_groups + p->mma8.size() +
                                           ((p->arbitrary.empty() && p->generic.empty() && p->copies.empty()) ? 0 : 1));
   if (ce == cudaSuccess) {

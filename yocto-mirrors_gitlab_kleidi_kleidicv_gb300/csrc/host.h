@@ -145,8 +145,17 @@ void *ctx_alloc(kleidicv_gpu_context *ctx, size_t bytes);
 void ctx_free(kleidicv_gpu_context *ctx, void *p, size_t bytes);
 // Copies `bytes` from host memory `src` to device memory `dst` on the
 // context's stream through the pinned upload ring: `src` may be reused as
-// soon as the call returns, and the call does not wait for earlier work.
+// soon as the call returns, and the call does not wait for earlier work unless
+// the ring's eight uploads before it are still outstanding: tables that go up
+// together are pieces of one upload, each at its offset from `dst` (the bytes
+// between them are overwritten too).
 cudaError_t upload_async(kleidicv_gpu_context *ctx, void *dst, const void *src, size_t bytes);
+struct UploadPiece {
+  size_t at;
+  const void *src;
+  size_t bytes;
+};
+cudaError_t upload_async(kleidicv_gpu_context *ctx, void *dst, const UploadPiece *pieces, size_t n);
 kleidicv_error_t cuda_status(kleidicv_gpu_context *ctx, cudaError_t e);
 
 // Device guard: makes ctx->device current for the calling thread.
