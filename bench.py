@@ -857,8 +857,8 @@ def _pyr_image(rng, w, h, c):
 
 def section_pyramid(torch, kcv, ctx, stream):
     """Seed 3: 8192x8192x1 and 4096x4096x3 through 5 blur_and_downsample
-    levels (REVERSE), each pyramid one launch; and 64 pyramids of 1024x768x4,
-    5 levels each, in one launch.  Source and level buffers rotate over sets
+    levels (REVERSE), a launch per level; and 64 pyramids of 1024x768x4, 5 levels
+    each, in one call (a launch per level of all of them).  Source and level buffers rotate over sets
     whose total exceeds twice the L2, so every call reads its level 0 from
     HBM.  Every level of the first set is compared with the CPU oracle."""
     from oracle import oracle
@@ -907,7 +907,7 @@ def section_pyramid(torch, kcv, ctx, stream):
                                "hbm_gbs": round(per_set / (ms * 1e-3) / 1e9, 1), "launches_per_pyramid": 5,
                                "rotating_sets": nsets, "all_levels_bit_exact": check(host, w, h, c, sets[0][1])}
         del sets
-    # 64 pyramids of 1024x768x4, 5 levels each: one launch.
+    # 64 pyramids of 1024x768x4, 5 levels each: one call.
     w, h, c = 1024, 768, 4
     sizes = levels_of(w, h)
     hosts = [_pyr_image(rng, w, h, c) for _ in range(64)]

@@ -131,8 +131,8 @@ struct Gauss8Job {
 };
 
 // u8 separable stencils on the tensor cores (csrc/mma8.cuh): generated
-// Gaussians of any size and the u8 separable filter.  A tile is 16 * MT
-// destination rows x tile_w destination bytes.
+// Gaussians of any size, the u8 separable filter and binomial 3x3 and 5x5.  A
+// tile is 16 * mt destination rows x tile_w destination bytes.
 struct Mma8Job {
   const uint8_t *src;
   uint8_t *dst;
@@ -144,7 +144,7 @@ struct Mma8Job {
   // Contraction steps: 16 source rows for 8 destination rows; 16 bytes of V
   // for destination bytes 8..15 (nb) and 0..7 (na) of 16.
   int32_t nk, nb, na;
-  int32_t mt, tile_w;     // a tile: 16 mt rows (1, 2, 4), destination bytes (a multiple of 128)
+  int32_t mt, tile_w;     // a tile: 16 mt rows (mt 2 or 4), destination bytes (256)
   int32_t epi;            // Mma8Epi
   int32_t tiles_x, tiles_y;
   int32_t raw_rows, raw_cols, raw_pitch;  // staged source: rows, bytes at a time, bytes between rows

@@ -235,8 +235,10 @@ __global__ void __launch_bounds__(128) median3_kernel(const uint8_t *src, int64_
 // and maxima per element (packed: two elements) at K = 5, where selecting from
 // each window by itself took 330.  Measured (1920x1080x1): u8 K = 5 / 7 49.4 /
 // 152 -> 12.1 / 26.5 us, f32 K = 5 49.4 -> 20.0 us; 160x120 K = 5 6.2 -> 3.8 us.
-// Bound by latency with few warps: half of the ALU pipe and 40 % of the issue
-// slots at 16 % of the warps resident (three blocks of up to 168 registers).  Four
+// Few warps and no full pipe: half of the ALU pipe and 40 % of the issue slots
+// at 16 % of the warps resident (three blocks of up to 168 registers).  Of a
+// warp's 6.3 cycles per instruction 1.8 are fixed waits between dependent
+// instructions, 0.7 global loads, 0.6 the ALU pipe, 0.4 shared memory.  Four
 // blocks of 128 registers spill: u8 1920x1080x3 K = 5 32.1 -> 28.3 us, but
 // 1280x720x1 5.6 -> 7.8 us and u16 1920x1080x1 11.9 -> 13.5 us.
 constexpr int median_width(int k) { return k == 7 ? 2 : 4; }  // pixels of a lane

@@ -59,10 +59,13 @@
 // 3840x2160x1 31 taps 132 -> 10.7 us, 255 taps 873 -> 77 us; 3840x2160x3 15
 // taps 66 -> 22.9 us, 1917x1079x3 (unaligned rows) 48.3 -> 13.9 us;
 // 3840x2160x4 21 taps 134 -> 43.1 us; 1920x1080x1 7 taps 9.3 -> 4.1 us.
-// Bound by latency at too few warps, not by a pipe: 3840x2160x1 at 7 / 31 /
-// 101 / 255 taps uses 44 / 42 / 34 / 33 % of the issue slots and 19 / 34 / 37 /
-// 43 % of the tensor pipe's cycles, with 25 % of the warps resident, and 14 %
-// (shared memory for one CTA) at 101 and 255 taps.  Three CTAs of 72
+// No pipe is full: 3840x2160x1 at 7 / 31 / 101 / 255 taps uses 44 / 42 / 34 /
+// 33 % of the issue slots and 19 / 34 / 37 / 43 % of the tensor pipe's cycles,
+// with 25 % of the warps resident, and 14 % (shared memory for one CTA) at 101
+// and 255 taps.  At 31 taps a warp takes 9.7 cycles per instruction: 1.9 in
+// fixed waits, 1.7 for the tensor pipe, 1.6 at the CTA's barriers, 0.7 for shared
+// memory, 0.65 for instructions, 0.4 for global loads; with unaligned rows
+// (1917x1079x3, 15 taps) 2.1 of 9.4 are for global loads and 1.0 at barriers.  Three CTAs of 72
 // registers per thread spill: 1920x1080x1 7 taps 4.9 us.  7 taps are 99 warp
 // instructions per 16 x 16 bytes; unaligned rows take 1.7 times as many.
 #pragma once

@@ -7,9 +7,10 @@
 
 namespace kcv {
 
-// Fills the job of a fused Gaussian with generated weights or a u8 separable
-// filter, or of an arbitrary-size Gaussian, tiled for `sm_count` SMs.  False:
-// the call is not of these kinds (or overlaps its source), and the job is not
+// Fills the job of a fused Gaussian with generated weights, a u8 separable
+// filter or a binomial 3x3 or 5x5 of a smaller or unaligned image, or of an
+// arbitrary-size Gaussian, tiled for `sm_count` SMs.  False: the call is not of
+// these kinds, or (arbitrary sizes) its images overlap, and the job is not
 // filled.
 bool mma8_job(const FilterJob &f, int sm_count, Mma8Job &j);
 bool mma8_job(const GenericJob &g, int sm_count, Mma8Job &j);
